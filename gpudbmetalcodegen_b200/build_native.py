@@ -46,6 +46,7 @@ HOST_SOURCES = [
 ]
 CUDA_SOURCES: list[str] = [
     "kernels/noalloc_distinct.cu",
+    "kernels/group_collect.cu",
     "kernels/sizer_mlp.cu",
     "kernels/batch_kernels.cu",
 ]

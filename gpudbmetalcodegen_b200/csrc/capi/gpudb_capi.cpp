@@ -613,7 +613,7 @@ int gpudb_ctx_sync(gpudb_ctx* ctx, unsigned* device_error) {
 int gpudb_result_shape(gpudb_result* r, int* ncols, long long* nrows) {
     if (!r) return GPUDB_E_INVALID;
     if (ncols) *ncols = (int)r->r.columns.size();
-    if (nrows) *nrows = (long long)r->r.rows.size();
+    if (nrows) *nrows = (long long)r->r.numRows();
     return GPUDB_OK;
 }
 
@@ -628,9 +628,10 @@ int gpudb_result_column(gpudb_result* r, int col, char* name, size_t cap, int* t
 }
 
 int gpudb_result_get_int(gpudb_result* r, long long row, int col, int64_t* lo, int64_t* hi) {
-    if (!r || row < 0 || row >= (long long)r->r.rows.size() || col < 0 || col >= (int)r->r.rows[row].size())
+    if (!r || row < 0 || row >= (long long)r->r.numRows() || col < 0 || col >= (int)r->r.columns.size())
         return GPUDB_E_INVALID;
-    const auto* v = std::get_if<gpudb::int128>(&r->r.rows[row][col]);
+    const auto cell = r->r.value(row, col);
+    const auto* v = std::get_if<gpudb::int128>(&cell);
     if (!v) return GPUDB_E_INVALID;
     if (lo) *lo = (int64_t)(unsigned long long)(*v);
     if (hi) *hi = (int64_t)(*v >> 64);
@@ -638,29 +639,40 @@ int gpudb_result_get_int(gpudb_result* r, long long row, int col, int64_t* lo, i
 }
 
 int gpudb_result_get_f64(gpudb_result* r, long long row, int col, double* out) {
-    if (!r || row < 0 || row >= (long long)r->r.rows.size() || col < 0 || col >= (int)r->r.rows[row].size())
+    if (!r || row < 0 || row >= (long long)r->r.numRows() || col < 0 || col >= (int)r->r.columns.size())
         return GPUDB_E_INVALID;
-    const auto* v = std::get_if<double>(&r->r.rows[row][col]);
+    const auto cell = r->r.value(row, col);
+    const auto* v = std::get_if<double>(&cell);
     if (!v) return GPUDB_E_INVALID;
     if (out) *out = *v;
     return GPUDB_OK;
 }
 
 size_t gpudb_result_get_str(gpudb_result* r, long long row, int col, char* buf, size_t cap) {
-    if (!r || row < 0 || row >= (long long)r->r.rows.size() || col < 0 || col >= (int)r->r.rows[row].size()) return 0;
-    const auto* v = std::get_if<std::string>(&r->r.rows[row][col]);
+    if (!r || row < 0 || row >= (long long)r->r.numRows() || col < 0 || col >= (int)r->r.columns.size()) return 0;
+    const auto cell = r->r.value(row, col);
+    const auto* v = std::get_if<std::string>(&cell);
     return v ? copyOut(*v, buf, cap) : 0;
 }
 
 int gpudb_result_export_i64(gpudb_result* r, int col, int64_t* out, long long n) {
-    if (!r || !out || col < 0 || col >= (int)r->r.columns.size() || n < (long long)r->r.rows.size())
+    if (!r || !out || col < 0 || col >= (int)r->r.columns.size() || n < (long long)r->r.numRows())
         return GPUDB_E_INVALID;
+    if (r->r.dense) {
+        std::memcpy(out, r->r.dense + (size_t)col * r->r.denseRows, r->r.denseRows * sizeof(int64_t));
+        return GPUDB_OK;
+    }
     for (size_t i = 0; i < r->r.rows.size(); i++) {
         const auto* v = std::get_if<gpudb::int128>(&r->r.rows[i][col]);
         if (!v || *v > (gpudb::int128)INT64_MAX || *v < (gpudb::int128)INT64_MIN) return GPUDB_E_INVALID;
         out[i] = (int64_t)*v;
     }
     return GPUDB_OK;
+}
+
+const int64_t* gpudb_result_column_data(gpudb_result* r, int col) {
+    if (!r || !r->r.dense || col < 0 || col >= (int)r->r.columns.size()) return nullptr;
+    return r->r.dense + (size_t)col * r->r.denseRows;
 }
 
 size_t gpudb_result_canonical(gpudb_result* r, int exact, char* buf, size_t cap) {

@@ -263,9 +263,53 @@ void CudaGenericExecutor::releaseAllocatedBuffers() {
     for (auto& [_, b] : buffers_)
         if (b.owned && b.ptr) cudaFree(b.ptr);
     buffers_.clear();
+    if (groupScratch_.dev) cudaFree(groupScratch_.dev);
+    groupScratch_.dev = nullptr;
+    groupScratch_.bytes = 0;
+}
+
+// The groups of a hash aggregate are compacted, ordered and made columns on
+// the device; where device scratch cannot be had the host walks the table.
+bool CudaGenericExecutor::collectGroupsOnDevice(const CudaResultSchema& schema, GenericResult& r) {
+    const auto& h = schema.hashAgg;
+    GroupTable t;
+    t.cap = resolver_.resolve(h.capacitySymbol);
+    t.keyBytes = h.keyType == "unsigned long long" ? 8 : 4;
+    t.packedStride = h.packedStride;
+    t.nAggs = (int)h.aggs.size();
+    auto buffer = [&](const std::string& name, size_t bytes) -> const void* {
+        size_t have = 0;
+        const void* p = bufferPtr(name, &have);
+        if (!p || have < bytes) throw std::runtime_error("collector: missing " + name);
+        return p;
+    };
+    const size_t slotBytes = t.packedStride > 0 ? 8 * (size_t)t.packedStride : (size_t)t.keyBytes;
+    t.keys = buffer(h.keyBuffer, t.cap * slotBytes);
+    if (t.packedStride <= 0) {
+        t.packedStride = 0;
+        for (const auto& a : h.aggs) t.aggs.push_back(buffer(a.buffer, t.cap * 8));
+    }
+    uint64_t rows = 0;
+    const int64_t* data = nullptr;
+    std::shared_ptr<HostBlock> host;
+    std::string error;
+    if (!collectGroups(t, h.sortByKey, groupScratch_, stream_, rows, data, host, error)) {
+        if (!error.empty()) throw std::runtime_error("collector: " + error);
+        return false;
+    }
+    r.columns.push_back({h.keyName, "int"});
+    for (const auto& a : h.aggs) r.columns.push_back({a.name, "int"});
+    r.dense = data;
+    r.denseRows = rows;
+    r.denseOwner = host;
+    return true;
 }
 
 GenericResult CudaGenericExecutor::collectResult(const CudaResultSchema& schema) {
+    if (schema.kind == CudaResultSchema::HASH_AGG) {
+        GenericResult r;
+        if (collectGroupsOnDevice(schema, r)) return r;
+    }
     return CudaResultCollector::collect(
         schema, [this](const std::string& n, void* dst, size_t bytes) { return readBuffer(n, dst, bytes); },
         [this](const std::string& e) { return resolver_.resolve(e); });

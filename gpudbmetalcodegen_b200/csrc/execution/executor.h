@@ -28,6 +28,7 @@
 #include <vector>
 
 #include "../core/cuda_codegen.h"
+#include "group_collect.h"
 #include "result_collector.h"
 #include "runtime_compiler.h"
 
@@ -106,6 +107,7 @@ public:
     void* bufferPtr(const std::string& name, size_t* bytes = nullptr) const;
     void releaseAllocatedBuffers();
     GenericResult collectResult(const CudaResultSchema& schema);
+    bool collectGroupsOnDevice(const CudaResultSchema& schema, GenericResult& r);
 
     cudaStream_t stream() const { return stream_; }
     int device() const { return device_; }
@@ -165,6 +167,7 @@ private:
     std::map<std::pair<uint64_t, CUfunction>, int> smemConfigured_;
     std::map<std::pair<uint64_t, CUfunction>, int> carveoutSet_;
     std::vector<cudaEvent_t> events_;
+    GroupWorkspace groupScratch_;  // device scratch of group collection, grown on demand
     struct GraphEntry {
         cudaGraph_t graph = nullptr;
         cudaGraphExec_t exec = nullptr;

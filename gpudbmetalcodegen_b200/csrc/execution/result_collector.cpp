@@ -1,5 +1,7 @@
 #include "result_collector.h"
 
+#include "group_collect.h"
+
 #include <algorithm>
 #include <cmath>
 #include <cstdio>
@@ -47,8 +49,8 @@ std::string serialise(const GenericResult& r, bool exact) {
     std::ostringstream o;
     for (size_t c = 0; c < r.columns.size(); c++) o << (c ? "," : "") << r.columns[c].name;
     o << "\n";
-    for (const auto& row : r.rows) {
-        for (size_t c = 0; c < row.size(); c++) o << (c ? "," : "") << fmt(row[c], exact);
+    for (size_t i = 0; i < r.numRows(); i++) {
+        for (size_t c = 0; c < r.columns.size(); c++) o << (c ? "," : "") << fmt(r.value(i, c), exact);
         o << "\n";
     }
     return o.str();
@@ -75,7 +77,7 @@ void GenericResult::print(int limit) const {
     int n = 0;
     while (std::getline(in, line)) {
         if (limit >= 0 && n > limit) {
-            std::cout << "... (" << rows.size() - (size_t)limit << " more rows)\n";
+            std::cout << "... (" << numRows() - (size_t)limit << " more rows)\n";
             break;
         }
         std::cout << line << "\n";
@@ -340,6 +342,37 @@ GenericResult CudaResultCollector::collectMaterialize(const CudaResultSchema& s,
     uint64_t cnt = 0;
     if (!read(s.counterBuffer, &cnt, 8)) throw std::runtime_error("collector: missing " + s.counterBuffer);
     for (const auto& c : s.columns) r.columns.push_back({c.displayName, c.elementType == "double" ? "double" : "int"});
+    bool ints = !s.columns.empty();  // every value fits an int64
+    for (const auto& c : s.columns) ints &= c.elementType != "double" && c.elementType != "unsigned long long";
+    if (ints) {
+        // columns, not rows: 64-bit ones are read into place, narrow ones widened
+        auto blk = hostBlock(s.columns.size() * cnt * 8);
+        auto* out = static_cast<int64_t*>(blk->ptr);
+        std::vector<char> raw;
+        for (size_t c = 0; c < s.columns.size() && cnt; c++, out += cnt) {
+            const std::string& t = s.columns[c].elementType;
+            const size_t w = cudaTypeBytes(t);
+            void* dst = out;
+            if (w != 8) {
+                raw.resize(cnt * w);
+                dst = raw.data();
+            }
+            if (!read(s.columns[c].bufferName, dst, cnt * w))
+                throw std::runtime_error("collector: missing " + s.columns[c].bufferName);
+            if (w == 8) continue;
+            const char* p = raw.data();
+            if (t == "unsigned" || t == "unsigned int")
+                for (uint64_t i = 0; i < cnt; i++) out[i] = reinterpret_cast<const uint32_t*>(p)[i];
+            else if (t == "unsigned char")
+                for (uint64_t i = 0; i < cnt; i++) out[i] = reinterpret_cast<const uint8_t*>(p)[i];
+            else
+                for (uint64_t i = 0; i < cnt; i++) out[i] = reinterpret_cast<const int32_t*>(p)[i];
+        }
+        r.dense = static_cast<const int64_t*>(blk->ptr);
+        r.denseRows = cnt;
+        r.denseOwner = blk;
+        return r;
+    }
     std::vector<std::vector<char>> cols;
     for (const auto& c : s.columns) {
         const size_t w = cudaTypeBytes(c.elementType);

@@ -14,6 +14,7 @@
 // ===================================================================
 #include <cstdint>
 #include <functional>
+#include <memory>
 #include <string>
 #include <variant>
 #include <vector>
@@ -33,14 +34,22 @@ struct GenericResult {
     using Value = std::variant<int128, double, std::string>;
     using Row = std::vector<Value>;
     std::vector<Row> rows;
+    // Large integer results as columns instead of rows (then `rows` is
+    // empty): column c at dense[c * denseRows], kept alive by denseOwner.
+    const int64_t* dense = nullptr;
+    size_t denseRows = 0;
+    std::shared_ptr<void> denseOwner;
+    Value value(size_t row, size_t col) const {
+        return dense ? Value((int128)dense[col * denseRows + row]) : rows[row][col];
+    }
 
     // Reference format: header line, CSV rows, doubles as %.4f.
     std::string toCanonical() const;
     // Full-precision variant used for exact parity (%.17g doubles).
     std::string toExact() const;
     void print(int limit = -1) const;
-    bool empty() const { return rows.empty(); }
-    size_t numRows() const { return rows.size(); }
+    bool empty() const { return numRows() == 0; }
+    size_t numRows() const { return dense ? denseRows : rows.size(); }
     int columnIndex(const std::string& name) const;
 };
 

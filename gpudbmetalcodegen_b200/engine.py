@@ -14,6 +14,7 @@ metal_generic_executor.cpp:91-93).
 from __future__ import annotations
 
 import ctypes as C
+import weakref
 from dataclasses import dataclass, field
 from typing import Any, Dict, Iterable, List, Mapping, Optional, Sequence
 
@@ -109,22 +110,47 @@ def _result_from_c(res) -> Result:
 
 
 def _arrays_from_c(res) -> Dict[str, np.ndarray]:
-    """Integer result columns as numpy int64 arrays (one bulk export per
-    column, no per-row Python objects) — for large results."""
+    """Integer result columns as numpy int64 arrays (no per-row Python
+    objects) — for large results. A result held as columns is handed over
+    without a copy: its arrays share the result's memory, which is freed
+    (or recycled) when the last of them is dropped. Takes over `res`."""
     lib = _lib.load()
     nc, nr = C.c_int(), C.c_longlong()
     lib.gpudb_result_shape(res, C.byref(nc), C.byref(nr))
-    out = {}
+    n = nr.value
+    names, types = [], []
     for c in range(nc.value):
         buf = C.create_string_buffer(256)
         t = C.c_int()
         lib.gpudb_result_column(res, c, buf, 256, C.byref(t))
-        if t.value != 0:
-            continue
-        a = np.zeros(nr.value, dtype=np.int64)
-        check(lib.gpudb_result_export_i64(res, c, a.ctypes.data, nr.value))
-        out[buf.value.decode()] = a
-    return out
+        names.append(buf.value.decode())
+        types.append(t.value)
+    ptr = lib.gpudb_result_column_data(res, 0) if nc.value and n else None
+    if ptr:
+        mem = (C.c_int64 * (nc.value * n)).from_address(ptr)
+        weakref.finalize(mem, lib.gpudb_result_free, C.c_void_p(res.value)).atexit = False
+        a = np.frombuffer(mem, dtype=np.int64)
+        return {name: a[c * n:(c + 1) * n] for c, name in enumerate(names)}
+    try:
+        out = {}
+        for c, (name, t) in enumerate(zip(names, types)):
+            if t != 0:
+                continue
+            a = np.zeros(n, dtype=np.int64)
+            check(lib.gpudb_result_export_i64(res, c, a.ctypes.data, n))
+            out[name] = a
+        return out
+    finally:
+        lib.gpudb_result_free(res)
+
+
+def _take_result(res, arrays: bool):
+    if arrays:
+        return _arrays_from_c(res)
+    try:
+        return _result_from_c(res)
+    finally:
+        _lib.load().gpudb_result_free(res)
 
 
 class Query:
@@ -327,10 +353,7 @@ class Context:
             raise err
         out = None
         if collect:
-            try:
-                out = _arrays_from_c(res) if arrays else _result_from_c(res)
-            finally:
-                self._lib.gpudb_result_free(res)
+            out = _take_result(res, arrays)
         return out, timing
 
     def run_streamed(self, spec_or_query, table: str, columns: Sequence[tuple], rows: int, chunk_rows: int,
@@ -356,10 +379,7 @@ class Context:
             raise GpudbError(st, _lib.last_error(self.handle))
         out = None
         if collect:
-            try:
-                out = _arrays_from_c(res) if arrays else _result_from_c(res)
-            finally:
-                self._lib.gpudb_result_free(res)
+            out = _take_result(res, arrays)
         return out, timing
 
     def collect(self, query: "Query") -> Result:
@@ -367,10 +387,7 @@ class Context:
         (e.g. the last of many enqueued graph replays), without running it."""
         res = C.c_void_p()
         check(self._lib.gpudb_query_collect(self.handle, query.handle, C.byref(res)), self.handle)
-        try:
-            return _result_from_c(res)
-        finally:
-            self._lib.gpudb_result_free(res)
+        return _take_result(res, False)
 
     def enqueue(self, spec_or_query, tune: str = "") -> None:
         """Enqueue one execution and return without waiting (no timing, no

@@ -108,6 +108,9 @@ size_t gpudb_result_get_str(gpudb_result* r, long long row, int col, char* buf, 
 /* Whole integer column as int64 (fails with GPUDB_E_INVALID if a value
  * does not fit). */
 int gpudb_result_export_i64(gpudb_result* r, int col, int64_t* out, long long n);
+/* A column of a result held as contiguous int64 columns (the groups of a
+ * hash aggregate), valid until the result is freed; NULL for other results. */
+const int64_t* gpudb_result_column_data(gpudb_result* r, int col);
 /* GenericResult::toCanonical (%.4f doubles) / full-precision variant. */
 size_t gpudb_result_canonical(gpudb_result* r, int exact, char* buf, size_t cap);
 void gpudb_result_free(gpudb_result* r);
