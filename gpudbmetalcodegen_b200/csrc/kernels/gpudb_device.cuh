@@ -320,6 +320,22 @@ __device__ __forceinline__ void gpudb_red_add_shared_u64(unsigned long long* p, 
     asm volatile("red.shared.add.u64 [%0], %1;" ::"r"(gpudb_smem_addr(p)), "l"(v) : "memory");
 }
 
+// ------------------------------------------------------------------
+// A 64-bit sum in shared memory, kept as two 32-bit words (lo, hi): the
+// low add returns the old word, whose wrap-around is the carry into hi, so
+// the pair is exact modulo 2^64 whatever the order of the adds. The
+// hardware adds 32-bit words in shared memory natively and 64-bit ones by a
+// compare-and-swap loop: on B200 a count plus a sum per row measured 272
+// against 1,571 G rows/s over 256 random slots, 24 against 783 over four
+// (lanes of a warp in one slot repeat the loop for each other).
+// ------------------------------------------------------------------
+__device__ __forceinline__ void gpudb_shared_add64(unsigned* lo, unsigned* hi, unsigned long long v) {
+    const unsigned vl = (unsigned)v;
+    const unsigned old = atomicAdd(lo, vl);
+    const unsigned h = (unsigned)(v >> 32) + (old + vl < vl ? 1u : 0u);
+    if (h) gpudb_red_add_shared_u32(hi, h);
+}
+
 __device__ __forceinline__ void gpudb_mbar_init(unsigned long long* bar, unsigned count) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(gpudb_smem_addr(bar)), "r"(count) : "memory");
 }

@@ -35,6 +35,22 @@ KeyOps keyOps(const std::string& keyType, HashLayout layout, bool packedOk = fal
     throw std::runtime_error("hash key type must be int or long long, got '" + keyType + "'");
 }
 
+bool isOne(const std::string& valueExpr) { return valueExpr == "1" || valueExpr == "1ll" || valueExpr == "1u"; }
+
+// Add `val` to sum j (of `slots` slots) of a shared-memory table whose sums
+// are (low, high) word pairs: low words at 2 j slots, high words at
+// (2 j + 1) slots. `unit`: val is 1 (a block sees fewer than 2^32 rows, so
+// the low word alone holds the count).
+std::string sharedAdd(const std::string& base, int j, int slots, const std::string& slot, const std::string& val, bool unit) {
+    const std::string lo = base + " + " + S(2ll * j * slots) + " + " + slot, hi = base + " + " + S((2ll * j + 1) * slots) + " + " + slot;
+    if (unit) return "gpudb_red_add_shared_u32(" + lo + ", 1u);";
+    return "gpudb_shared_add64(" + lo + ", " + hi + ", (unsigned long long)" + val + ");";
+}
+std::string sharedSum(const std::string& base, int j, int slots, const std::string& slot) {
+    return "(((unsigned long long)" + base + "[" + S((2ll * j + 1) * slots) + " + " + slot + "] << 32) | " + base + "[" +
+           S(2ll * j * slots) + " + " + slot + "])";
+}
+
 // Bucket8 probes count buckets of 8 slots; keep the same slot budget.
 int probeArg(HashLayout layout, int maxProbe) {
     return layout == HashLayout::Bucket8 ? (maxProbe + 7) / 8 : maxProbe;
@@ -919,7 +935,7 @@ void CudaKeyedAgg::produce(CudaCodegen& cg, ConsumerFn consume) {
         std::vector<int> pos(na, 0);
         for (int j = 0; j < na; j++) {
             const std::string& v = aggregates_[j].valueExpr;
-            narrow[j] = (v == "1" || v == "1ll" || v == "1u");
+            narrow[j] = isOne(v);
             pos[j] = narrow[j] ? nNarrow++ : nWide++;
         }
         const int accW = nb * nWide, accN = nb * nNarrow;
@@ -983,27 +999,29 @@ void CudaKeyedAgg::produce(CudaCodegen& cg, ConsumerFn consume) {
     } else if (st == Strategy::Shared) {
         const int words = nb * vpb;
         const int soff = cg.allocDynamicSmem(words * 8);
-        cg.addComment("keyed aggregation: per-block shared-memory table of " + S(words) + " words");
-        cg.addLine("unsigned long long* _ks = reinterpret_cast<unsigned long long*>(gpudb_smem + " + S(soff) + ");");
-        cg.addLine("for (int _w = threadIdx.x; _w < " + S(words) + "; _w += blockDim.x) _ks[_w] = 0ull;");
+        cg.addComment("keyed aggregation: per-block shared-memory table of " + S(words) + " words, as (low, high) words");
+        cg.addLine("unsigned* _ks = reinterpret_cast<unsigned*>(gpudb_smem + " + S(soff) + ");");
+        cg.addLine("for (int _w = threadIdx.x; _w < " + S(2 * words) + "; _w += blockDim.x) _ks[_w] = 0u;");
         cg.addLine("__syncthreads();");
         child_->produce(cg, [&]() {
             emitValues();
             cg.addBlock("if ((unsigned)_bucket < " + S(nb) + "u)", [&]() {
                 for (int j = 0; j < na; j++) {
                     const auto& ag = aggregates_[j];
-                    const std::string base = "_ks + _bucket * " + S(vpb) + " + " + S(ag.offset);
-                    if (ag.isWide)
-                        cg.addLine("gpudb_acc128_add(" + base + ", _kv" + S(j) + ");");
-                    else
-                        cg.addLine("atomicAdd(" + base + ", (unsigned long long)_kv" + S(j) + ");");
+                    const std::string at = "_bucket * " + S(vpb) + " + " + S(ag.offset), v = "_kv" + S(j);
+                    if (ag.isWide) {  // the two words of gpudb_acc128_add
+                        cg.addLine(sharedAdd("_ks", 0, words, at, "(" + v + " & 0xFFFFFFFFll)", false));
+                        cg.addLine(sharedAdd("_ks", 0, words, at + " + 1", "(" + v + " >> 32)", false));
+                    } else {
+                        cg.addLine(sharedAdd("_ks", 0, words, at, v, isOne(ag.valueExpr)));
+                    }
                 }
             }, " else { gpudb_set_error(gpudb_err, GPUDB_ERR_BOUNDS); }");
             consume();
         });
         cg.addLine("__syncthreads();");
         cg.addBlock("for (int _w = threadIdx.x; _w < " + S(words) + "; _w += blockDim.x)", [&]() {
-            cg.addLine("const unsigned long long _v = _ks[_w];");
+            cg.addLine("const unsigned long long _v = " + sharedSum("_ks", 0, words, "_w") + ";");
             cg.addLine("if (_v != 0ull) atomicAdd(" + out + " + _w, _v);");
         });
     } else {
@@ -1071,9 +1089,9 @@ void CudaAtomicAgg::produce(CudaCodegen& cg, ConsumerFn consume) {
         const int vo = cg.allocDynamicSmem(slots * 8 * na);
         cg.addComment("per-block shared-memory cache of hot buckets (" + S(slots) + " slots)");
         cg.addLine("unsigned long long* _ac_k = reinterpret_cast<unsigned long long*>(gpudb_smem + " + S(ko) + ");");
-        cg.addLine("unsigned long long* _ac_v = reinterpret_cast<unsigned long long*>(gpudb_smem + " + S(vo) + ");");
+        cg.addLine("unsigned* _ac_v = reinterpret_cast<unsigned*>(gpudb_smem + " + S(vo) + ");  // (low, high) words");
         cg.addLine("for (int _w = threadIdx.x; _w < " + S(slots) + "; _w += blockDim.x) _ac_k[_w] = GPUDB_EMPTY64;");
-        cg.addLine("for (int _w = threadIdx.x; _w < " + S(slots * na) + "; _w += blockDim.x) _ac_v[_w] = 0ull;");
+        cg.addLine("for (int _w = threadIdx.x; _w < " + S(2 * slots * na) + "; _w += blockDim.x) _ac_v[_w] = 0u;");
         cg.addLine("__syncthreads();");
     }
     child_->produce(cg, [&]() {
@@ -1089,7 +1107,7 @@ void CudaAtomicAgg::produce(CudaCodegen& cg, ConsumerFn consume) {
                            S(smemProbe_) + ");");
                 cg.addBlock("if (_as >= 0)", [&]() {
                     for (int j = 0; j < na; j++)
-                        cg.addLine("atomicAdd(_ac_v + " + S(j * slots) + " + _as, (unsigned long long)_av" + S(j) + ");");
+                        cg.addLine(sharedAdd("_ac_v", j, slots, "_as", "_av" + S(j), !warpAgg_ && isOne(arrs[j].second)));
                 }, " else {");
                 cg.increaseIndent();
                 for (int j = 0; j < na; j++)
@@ -1106,7 +1124,9 @@ void CudaAtomicAgg::produce(CudaCodegen& cg, ConsumerFn consume) {
         if (warpAgg_) {
             cg.addLine("const unsigned _am = __activemask();");
             cg.addLine("const unsigned _peers = __match_any_sync(_am, (unsigned long long)_ab);");
-            for (int j = 0; j < na; j++) cg.addLine("_av" + S(j) + " = gpudb_peer_sum(_am, _peers, _av" + S(j) + ");");
+            for (int j = 0; j < na; j++)
+                cg.addLine("_av" + S(j) + " = " + (isOne(arrs[j].second) ? "(long long)__popc(_peers);" :
+                           "gpudb_peer_sum(_am, _peers, _av" + S(j) + ");"));
             cg.addIf("(int)(threadIdx.x & 31u) == __ffs(_peers) - 1", update);
         } else {
             update();
@@ -1118,9 +1138,11 @@ void CudaAtomicAgg::produce(CudaCodegen& cg, ConsumerFn consume) {
         cg.addBlock("for (int _w = threadIdx.x; _w < " + S(slots) + "; _w += blockDim.x)", [&]() {
             cg.addLine("const unsigned long long _k = _ac_k[_w];");
             cg.addLine("if (_k == GPUDB_EMPTY64) continue;");
-            for (int j = 0; j < na; j++)
-                cg.addLine("if (_ac_v[" + S(j * slots) + " + _w] != 0ull) atomicAdd(" + arrs[j].first + " + _k, _ac_v[" +
-                           S(j * slots) + " + _w]);");
+            for (int j = 0; j < na; j++) {
+                const std::string v = "_as" + S(j);
+                cg.addLine("const unsigned long long " + v + " = " + sharedSum("_ac_v", j, slots, "_w") + ";");
+                cg.addLine("if (" + v + " != 0ull) atomicAdd(" + arrs[j].first + " + _k, " + v + ");");
+            }
         });
     }
 }
@@ -1436,12 +1458,13 @@ void CudaHashGroupBy::produce(CudaCodegen& cg, ConsumerFn consume) {
         const int slots = 1 << L;
         const int ko_off = cg.allocDynamicSmem(slots * 8);
         const int vo_off = cg.allocDynamicSmem(slots * 8 * na);
-        cg.addComment("per-block shared-memory pre-aggregation table (" + S(slots) + " slots) for heavy hitters");
+        cg.addComment("per-block shared-memory pre-aggregation table (" + S(slots) +
+                      " slots) for heavy hitters; sums as (low, high) words");
         cg.addLine("unsigned long long* _gs_k = reinterpret_cast<unsigned long long*>(gpudb_smem + " + S(ko_off) + ");");
-        cg.addLine("unsigned long long* _gs_v = reinterpret_cast<unsigned long long*>(gpudb_smem + " + S(vo_off) + ");");
+        cg.addLine("unsigned* _gs_v = reinterpret_cast<unsigned*>(gpudb_smem + " + S(vo_off) + ");");
         cg.addBlock("for (int _w = threadIdx.x; _w < " + S(slots) + "; _w += blockDim.x)", [&]() {
             cg.addLine("_gs_k[_w] = GPUDB_EMPTY64;");
-            for (int j = 0; j < na; j++) cg.addLine("_gs_v[" + S(j) + " * " + S(slots) + " + _w] = 0ull;");
+            for (int j = 0; j < 2 * na; j++) cg.addLine("_gs_v[" + S(j * slots) + " + _w] = 0u;");
         });
         cg.addLine("__syncthreads();");
     }
@@ -1492,6 +1515,8 @@ void CudaHashGroupBy::produce(CudaCodegen& cg, ConsumerFn consume) {
         cg.decreaseIndent();
         cg.addLine("}");
     };
+    // a count of rows that no warp aggregation has summed: always 1
+    auto unitAgg = [&](int j) { return !warpAgg_ && isOne(aggs_[j].valueExpr); };
     child_->produce(cg, [&]() {
         cg.addLine("const long long _gk = (long long)(" + keyExpr_ + ");");
         std::vector<std::string> vals;
@@ -1504,9 +1529,7 @@ void CudaHashGroupBy::produce(CudaCodegen& cg, ConsumerFn consume) {
                 cg.addLine("const int _gss = gpudb_smem_ht_slot64(_gs_k, " + S(L) + ", (unsigned long long)_gk, " +
                            S(smemProbe_) + ");");
                 cg.addBlock("if (_gss >= 0)", [&]() {
-                    for (int j = 0; j < na; j++)
-                        cg.addLine("atomicAdd(_gs_v + " + S(j) + " * " + S(1 << L) + " + _gss, (unsigned long long)_gv" +
-                                   S(j) + ");");
+                    for (int j = 0; j < na; j++) cg.addLine(sharedAdd("_gs_v", j, 1 << L, "_gss", "_gv" + S(j), unitAgg(j)));
                 }, " else {");
                 cg.increaseIndent();
                 globalUpdate("(_gk)", vals);
@@ -1519,7 +1542,9 @@ void CudaHashGroupBy::produce(CudaCodegen& cg, ConsumerFn consume) {
         if (warpAgg_) {
             cg.addLine("const unsigned _gm = __activemask();");
             cg.addLine("const unsigned _gpeers = __match_any_sync(_gm, (unsigned long long)_gk);");
-            for (int j = 0; j < na; j++) cg.addLine("_gv" + S(j) + " = gpudb_peer_sum(_gm, _gpeers, _gv" + S(j) + ");");
+            for (int j = 0; j < na; j++)
+                cg.addLine("_gv" + S(j) + " = " + (isOne(aggs_[j].valueExpr) ? "(long long)__popc(_gpeers);" :
+                           "gpudb_peer_sum(_gm, _gpeers, _gv" + S(j) + ");"));
             cg.addIf("(int)(threadIdx.x & 31u) == __ffs(_gpeers) - 1", update);
         } else {
             update();
@@ -1533,7 +1558,7 @@ void CudaHashGroupBy::produce(CudaCodegen& cg, ConsumerFn consume) {
             cg.addLine("const unsigned long long _fk = _gs_k[_w];");
             cg.addLine("if (_fk == GPUDB_EMPTY64) continue;");
             std::vector<std::string> vals;
-            for (int j = 0; j < na; j++) vals.push_back("_gs_v[" + S(j) + " * " + S(1 << L) + " + _w]");
+            for (int j = 0; j < na; j++) vals.push_back(sharedSum("_gs_v", j, 1 << L, "_w"));
             globalUpdate("(_fk)", vals);
         });
     }
@@ -1606,6 +1631,72 @@ void CudaHashWarmFlush::produce(CudaCodegen& cg, ConsumerFn consume) {
 
 std::string CudaHashWarmFlush::describe() const {
     return "HashWarmFlush(" + table_ + ", " + S(1ll << warmLog2_) + " warm slots)";
+}
+
+// ===================================================================
+// CudaHashCompact
+// ===================================================================
+CudaHashCompact::CudaHashCompact(const std::string& tableName, const std::string& capacityExpr,
+                                 const std::vector<std::string>& aggNames, const std::string& outPrefix,
+                                 const std::string& outCapacityExpr)
+    : table_(tableName), capExpr_(capacityExpr), aggs_(aggNames), out_(outPrefix), outCap_(outCapacityExpr) {}
+
+void CudaHashCompact::produce(CudaCodegen& cg, ConsumerFn consume) {
+    const std::string n = out_ + "_n", slots = "n_" + table_ + "_slots";
+    cg.addReadBufferParam(table_ + "_keys", "unsigned long long");
+    for (const auto& a : aggs_) cg.addReadBufferParam(table_ + "_" + a, "unsigned long long");
+    cg.addSizeScalarParam(slots, "long long", hashSlotsExpr(capExpr_));
+    cg.addAtomicBufferParam(n, "unsigned long long", "1");
+    cg.addBufferParam(out_ + "_key", "long long", outCap_, false);
+    for (const auto& a : aggs_) cg.addBufferParam(out_ + "_" + a, "long long", outCap_, false);
+    cg.addSizeScalarParam("cap_" + n, "long long", outCap_);
+    cg.addComment("the created groups of " + table_ + ", dense: four slots per thread, one position atomic per CTA round");
+    cg.addLine("__shared__ unsigned _hc_w[32];");
+    cg.addLine("__shared__ unsigned long long _hc_base;");
+    cg.addLine("const int _hc_nw = (int)(blockDim.x >> 5);");
+    cg.addBlock("for (long long _hb = (long long)blockIdx.x * blockDim.x * 4; _hb < " + slots +
+                    "; _hb += (long long)gridDim.x * blockDim.x * 4)",
+                [&]() {
+        cg.addLine("unsigned long long _hk[4];");
+        cg.addLine("unsigned _hm = 0u;");
+        cg.addLine("#pragma unroll");
+        cg.addBlock("for (int _u = 0; _u < 4; ++_u)", [&]() {
+            cg.addLine("const long long _s = _hb + _u * (int)blockDim.x + (int)threadIdx.x;");
+            cg.addLine("_hk[_u] = _s < " + slots + " ? __ldg(" + table_ + "_keys + _s) : GPUDB_EMPTY64;");
+            cg.addLine("_hm |= _hk[_u] != GPUDB_EMPTY64 ? 1u << _u : 0u;");
+        });
+        cg.addLine("unsigned _hx = __popc(_hm);");
+        cg.addLine("#pragma unroll");
+        cg.addBlock("for (int _o = 1; _o < 32; _o <<= 1)", [&]() {
+            cg.addLine("const unsigned _y = __shfl_up_sync(0xffffffffu, _hx, _o);");
+            cg.addLine("if (simd_lane >= (unsigned)_o) _hx += _y;");
+        });
+        cg.addLine("if (simd_lane == 31u) _hc_w[simd_id] = _hx;");
+        cg.addLine("__syncthreads();");
+        cg.addBlock("if (threadIdx.x == 0u)", [&]() {
+            cg.addLine("unsigned _t = 0u;");
+            cg.addLine("for (int _w = 0; _w < _hc_nw; ++_w) { const unsigned _c = _hc_w[_w]; _hc_w[_w] = _t; _t += _c; }");
+            cg.addLine("_hc_base = _t ? atomicAdd(" + n + ", (unsigned long long)_t) : 0ull;");
+        });
+        cg.addLine("__syncthreads();");
+        cg.addLine("unsigned long long _p = _hc_base + _hc_w[simd_id] + _hx - __popc(_hm);");
+        cg.addLine("#pragma unroll");
+        cg.addBlock("for (int _u = 0; _u < 4; ++_u)", [&]() {
+            cg.addLine("if (!(_hm >> _u & 1u)) continue;");
+            cg.addLine("const long long _s = _hb + _u * (int)blockDim.x + (int)threadIdx.x;");
+            cg.addBlock("if (_p < (unsigned long long)cap_" + n + ")", [&]() {
+                cg.addLine(out_ + "_key[_p] = (long long)_hk[_u];");
+                for (const auto& a : aggs_) cg.addLine(out_ + "_" + a + "[_p] = (long long)" + table_ + "_" + a + "[_s];");
+            }, " else { gpudb_set_error(gpudb_err, GPUDB_ERR_CAPACITY); }");
+            cg.addLine("++_p;");
+        });
+        cg.addLine("__syncthreads();");
+    });
+    consume();
+}
+
+std::string CudaHashCompact::describe() const {
+    return "HashCompact(" + table_ + " -> " + out_ + ", " + S(1 + (long long)aggs_.size()) + " columns)";
 }
 
 // ===================================================================

@@ -724,22 +724,13 @@ CudaQueryPlan buildGroupBySorted(Spec& s, const TuneConfig& tune) {
         gb->addAggregate("sum", "z_value[i]");
         gb->setWarpAggregate(tune.warpAggregate);
         gb->setSharedPreAgg(tune.smemPreAggLog2, tune.smemProbe);
-        gb->setSlotList(true);
         appendPhase(plan, "GS_group", std::move(gb), tune);
     }
     const std::string cap = "max(" + groupsExpr + ", 1)";
-    {
-        auto ls = std::make_unique<CudaSlotListScan>("gs_slotlist", "gs_nslots");
-        auto mt = std::make_unique<CudaMaterialize>(std::move(ls), "gsc_n", cap);
-        mt->addColumn("gsc_key", "long long", "(long long)gs_keys[i]");
-        mt->addColumn("gsc_count", "long long", "(long long)gs_count[i]");
-        mt->addColumn("gsc_sum", "long long", "(long long)gs_sum[i]");
-        mt->setIntermediate(true);
-        auto& ph = appendPhase(plan, "GS_compact", std::move(mt), tune);
-        ph.extraBuffers.push_back({"gs_keys", "unsigned long long", true, false});
-        ph.extraBuffers.push_back({"gs_count", "unsigned long long", true, false});
-        ph.extraBuffers.push_back({"gs_sum", "unsigned long long", true, false});
-    }
+    appendPhase(plan, "GS_compact",
+                std::make_unique<CudaHashCompact>("gs", hashCapacity(groupsExpr, tune),
+                                                  std::vector<std::string>{"count", "sum"}, "gsc", cap),
+                tune);
     TuneConfig st = tune;
     st.blockSize = 512;
     st.minBlocksPerSM = 1;
