@@ -95,6 +95,7 @@ void CudaCodegen::setPhaseThreadgroupSize(int s) {
 }
 void CudaCodegen::setPhaseSingleThread(bool s) { cur("setPhaseSingleThread").isSingleThread = s; }
 void CudaCodegen::setPhaseMaxThreadgroups(int m) { cur("setPhaseMaxThreadgroups").maxThreadgroups = m; }
+void CudaCodegen::setPhaseCooperative(bool on) { cur("setPhaseCooperative").cooperative = on; }
 void CudaCodegen::setPhaseDynamicSmem(int b) { cur("setPhaseDynamicSmem").dynamicSmemBytes = b; }
 void CudaCodegen::setPhaseTileRows(int r) { cur("setPhaseTileRows").tileRows = r; }
 void CudaCodegen::setPhaseRowsPerThread(int r) { cur("setPhaseRowsPerThread").rowsPerThread = r > 0 ? r : 1; }

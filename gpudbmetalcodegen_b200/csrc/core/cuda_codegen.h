@@ -76,6 +76,7 @@ public:
     void setPhaseThreadgroupSize(int size);
     void setPhaseSingleThread(bool single);
     void setPhaseMaxThreadgroups(int max);
+    void setPhaseCooperative(bool on);
     void setPhaseDynamicSmem(int bytes);
     void setPhaseTileRows(int rows);
     void setPhaseRowsPerThread(int rows);
@@ -135,6 +136,7 @@ public:
         std::string scannedTable;
         int threadgroupSize = 256;
         int maxThreadgroups = 0;
+        bool cooperative = false;  // the blocks wait on one another: launched all resident
         bool isSingleThread = false;
         int dynamicSmemBytes = 0;
         int tileRows = 0;

@@ -29,6 +29,7 @@ const DriverApi& driverApi() {
                   fetch(api, "cuModuleUnload", api.cuModuleUnload) &&
                   fetch(api, "cuModuleGetFunction", api.cuModuleGetFunction) &&
                   fetch(api, "cuLaunchKernel", api.cuLaunchKernel) &&
+                  fetch(api, "cuLaunchCooperativeKernel", api.cuLaunchCooperativeKernel) &&
                   fetch(api, "cuFuncSetAttribute", api.cuFuncSetAttribute) &&
                   fetch(api, "cuFuncGetAttribute", api.cuFuncGetAttribute) &&
                   fetch(api, "cuOccupancyMaxActiveBlocksPerMultiprocessor",

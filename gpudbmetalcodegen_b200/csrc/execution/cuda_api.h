@@ -19,6 +19,8 @@ struct DriverApi {
     CUresult (*cuModuleGetFunction)(CUfunction*, CUmodule, const char*) = nullptr;
     CUresult (*cuLaunchKernel)(CUfunction, unsigned, unsigned, unsigned, unsigned, unsigned, unsigned, unsigned,
                                CUstream, void**, void**) = nullptr;
+    CUresult (*cuLaunchCooperativeKernel)(CUfunction, unsigned, unsigned, unsigned, unsigned, unsigned, unsigned,
+                                          unsigned, CUstream, void**) = nullptr;
     CUresult (*cuFuncSetAttribute)(CUfunction, CUfunction_attribute, int) = nullptr;
     CUresult (*cuFuncGetAttribute)(int*, CUfunction_attribute, CUfunction) = nullptr;
     CUresult (*cuOccupancyMaxActiveBlocksPerMultiprocessor)(int*, CUfunction, int, size_t) = nullptr;

@@ -340,6 +340,7 @@ bool CudaGenericExecutor::buildLaunch(const RuntimeCompiler::CompiledQuery& cq, 
     l.name = ph.name;
     l.block = ph.isSingleThread ? 1u : (unsigned)ph.threadgroupSize;
     l.smem = (unsigned)ph.dynamicSmemBytes;
+    l.cooperative = ph.cooperative;
     const std::pair<uint64_t, CUfunction> fkey{cq.loadId, l.fn};
     auto sc = smemConfigured_.find(fkey);
     // any dynamic shared memory gets the opt-in: 48 KB of it plus the
@@ -533,7 +534,9 @@ int CudaGenericExecutor::execute(const RuntimeCompiler::CompiledQuery& cq,
             for (size_t k = 0; k < l.slots.size(); k++) args[k] = &l.slots[k];
             if (timed) cudaEventRecord(events_[2 * i], stream_);
             const CUresult r =
-                api.cuLaunchKernel(l.fn, l.grid, 1, 1, l.block, 1, 1, l.smem, (CUstream)stream_, args.data(), nullptr);
+                l.cooperative
+                    ? api.cuLaunchCooperativeKernel(l.fn, l.grid, 1, 1, l.block, 1, 1, l.smem, (CUstream)stream_, args.data())
+                    : api.cuLaunchKernel(l.fn, l.grid, 1, 1, l.block, 1, 1, l.smem, (CUstream)stream_, args.data(), nullptr);
             if (r != CUDA_SUCCESS) {
                 error = "launch of '" + l.name + "' failed: " + cuErrorString(r);
                 return false;

@@ -137,6 +137,7 @@ private:
     struct Launch {
         CUfunction fn;
         unsigned grid, block, smem;
+        bool cooperative;
         std::vector<uint64_t> slots;
         std::string name;
     };

@@ -165,50 +165,6 @@ __device__ __forceinline__ bool gpudb_row_before(long long va, long long ka, lon
     return va > vb || (va == vb && ka < kb);
 }
 
-// Merge passes a sort of n rows in chunks of `chunk` rows needs: the
-// smallest q with chunk << q >= n.
-__device__ __forceinline__ int gpudb_merge_passes(long long n, int chunk) {
-    int q = 0;
-    while (((long long)chunk << q) < n) q++;
-    return q;
-}
-
-// The same split found by one warp together: each round its 32 lanes test
-// 32 evenly spaced candidates (the test is monotone: true for every index
-// below the split), so the range shrinks 32-fold per round of loads. All
-// lanes of the warp call it and get the split.
-__device__ __forceinline__ int gpudb_merge_path_warp(const long long* av, const long long* ak, int na,
-                                                     const long long* bv, const long long* bk, int nb, int d) {
-    const int lane = (int)(threadIdx.x & 31u);
-    int lo = d > nb ? d - nb : 0, hi = d < na ? d : na;
-    while (lo < hi) {
-        const int step = (hi - lo + 31) / 32;
-        const int i = lo + lane * step;
-        const bool t = i < hi && !gpudb_row_before(bv[d - 1 - i], bk[d - 1 - i], av[i], ak[i]);
-        const int c = __popc(__ballot_sync(0xffffffffu, t));
-        if (c == 0) break;  // the split is lo
-        const int nlo = lo + (c - 1) * step + 1, nhi = lo + c * step;
-        lo = nlo;
-        hi = nhi < hi ? nhi : hi;
-    }
-    return lo;
-}
-
-// Merge path split of diagonal d between sorted A[0..na) and B[0..nb)
-// (arrays of value / key, row order gpudb_row_before): the number of A rows
-// among the first d merged rows (ties take A first).
-__device__ __forceinline__ int gpudb_merge_path(const long long* av, const long long* ak, int na, const long long* bv,
-                                                const long long* bk, int nb, int d) {
-    int lo = d > nb ? d - nb : 0, hi = d < na ? d : na;
-    while (lo < hi) {
-        const int mid = (lo + hi) >> 1;
-        // A[mid] goes before B[d - 1 - mid]: more A rows belong to the prefix
-        if (!gpudb_row_before(bv[d - 1 - mid], bk[d - 1 - mid], av[mid], ak[mid])) lo = mid + 1;
-        else hi = mid;
-    }
-    return lo;
-}
-
 // ------------------------------------------------------------------
 // Bitmaps (semi / anti joins). Reference: bitmap_test / bitmap_set,
 // metal_common_header.h:103-111.
@@ -652,6 +608,182 @@ __device__ __forceinline__ int gpudb_smem_ht_slot64(unsigned long long* skeys, i
         s = (s + 1u) & mask;
     }
     return -1;
+}
+
+// ------------------------------------------------------------------
+// Sorting inside one cooperative kernel: every block is resident, so the
+// passes of a radix sort follow each other through a grid barrier instead
+// of kernel boundaries, and their number is decided on the device.
+// ------------------------------------------------------------------
+// All blocks meet; `bar` counts arrivals from zero and `epoch` is the
+// caller's number of barriers so far. False (error word set) when the wait
+// runs out. Called by every thread.
+__device__ __forceinline__ bool gpudb_grid_barrier(unsigned* bar, unsigned& epoch, unsigned* err) {
+    __syncthreads();
+    ++epoch;
+    bool ok = true;
+    if (threadIdx.x == 0) {
+        __threadfence();
+        atomicAdd(bar, 1u);
+        const unsigned want = epoch * gridDim.x;
+        const unsigned long long t0 = gpudb_now_ns();
+        unsigned seen;
+        for (;;) {
+            asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(bar) : "memory");
+            if ((int)(seen - want) >= 0) break;
+            if (gpudb_now_ns() - t0 > GPUDB_WAIT_NS) {
+                gpudb_set_error(err, GPUDB_ERR_WAIT_TIMEOUT);
+                ok = false;
+                break;
+            }
+        }
+        __threadfence();
+    }
+    return !__syncthreads_or(!ok);
+}
+
+// Least-significant-digit radix sort of (64-bit key, 32-bit index) pairs,
+// 8-bit digits, tiles of 4096. One pass is count -> barrier -> scan ->
+// barrier -> scatter -> barrier. What another block wrote in this kernel is
+// read through L2 (__ldcg). Blocks of GPUDB_RS_THREADS threads.
+#define GPUDB_RS_THREADS 512
+#define GPUDB_RS_WARPS (GPUDB_RS_THREADS / 32)
+#define GPUDB_RS_ITEMS 8
+#define GPUDB_RS_TILE (GPUDB_RS_THREADS * GPUDB_RS_ITEMS)
+#define GPUDB_RS_SMEM_WORDS (GPUDB_RS_WARPS * 256 + 256 + 32)
+
+// counts[digit * ntiles + tile]
+__device__ __forceinline__ void gpudb_rs_count(const unsigned long long* k, unsigned n, int shift, unsigned* counts,
+                                               unsigned ntiles, unsigned* sh) {
+    for (unsigned t = blockIdx.x; t < ntiles; t += gridDim.x) {
+        for (int d = (int)threadIdx.x; d < 256; d += GPUDB_RS_THREADS) sh[d] = 0u;
+        __syncthreads();
+#pragma unroll
+        for (int u = 0; u < GPUDB_RS_ITEMS; ++u) {
+            const unsigned i = t * GPUDB_RS_TILE + u * GPUDB_RS_THREADS + threadIdx.x;
+            if (i < n) atomicAdd(sh + ((unsigned)(__ldcg(k + i) >> shift) & 255u), 1u);
+        }
+        __syncthreads();
+        for (int d = (int)threadIdx.x; d < 256; d += GPUDB_RS_THREADS) counts[(unsigned)d * ntiles + t] = sh[d];
+        __syncthreads();
+    }
+}
+
+// Exclusive block-wide prefix of one word per thread; *total gets the sum.
+__device__ __forceinline__ unsigned gpudb_rs_block_scan(unsigned v, unsigned* sw, unsigned* total) {
+    const unsigned lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    unsigned x = v;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const unsigned y = __shfl_up_sync(0xffffffffu, x, o);
+        if ((int)lane >= o) x += y;
+    }
+    if (lane == 31u) sw[warp] = x;
+    __syncthreads();
+    unsigned before = 0u, all = 0u;
+#pragma unroll
+    for (unsigned w = 0; w < GPUDB_RS_WARPS; ++w) {
+        const unsigned c = sw[w];
+        before += w < warp ? c : 0u;
+        all += c;
+    }
+    __syncthreads();
+    *total = all;
+    return before + x - v;
+}
+
+// A digit's tile counts become exclusive prefixes; its total is totals[digit].
+__device__ __forceinline__ void gpudb_rs_scan(unsigned* counts, unsigned ntiles, unsigned* totals, unsigned* sw) {
+    for (unsigned d = blockIdx.x; d < 256u; d += gridDim.x) {
+        unsigned* c = counts + d * ntiles;
+        unsigned carry = 0u;
+        for (unsigned b = 0; b < ntiles; b += GPUDB_RS_THREADS) {
+            const unsigned i = b + threadIdx.x;
+            unsigned all;
+            const unsigned p = gpudb_rs_block_scan(i < ntiles ? __ldcg(c + i) : 0u, sw, &all);
+            if (i < ntiles) c[i] = carry + p;
+            carry += all;
+        }
+        if (threadIdx.x == 0) totals[d] = carry;
+    }
+}
+
+// Stable scatter: a warp owns GPUDB_RS_ITEMS * 32 consecutive pairs of a
+// tile and ranks equal digits by match-any, 32 at a time.
+__device__ __forceinline__ void gpudb_rs_scatter(const unsigned long long* kin, const unsigned* xin, unsigned n, int shift,
+                                                 const unsigned* counts, const unsigned* totals, unsigned ntiles,
+                                                 unsigned long long* kout, unsigned* xout, unsigned* sh) {
+    const unsigned lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    unsigned* cnt = sh;                                // [warp][digit]
+    unsigned* base = sh + GPUDB_RS_WARPS * 256;        // the digits' first positions
+    unsigned* sw = base + 256;
+    unsigned all;
+    const unsigned first = gpudb_rs_block_scan(threadIdx.x < 256u ? __ldcg(totals + threadIdx.x) : 0u, sw, &all);
+    if (threadIdx.x < 256u) base[threadIdx.x] = first;
+    for (unsigned t = blockIdx.x; t < ntiles; t += gridDim.x) {
+        for (int w = (int)threadIdx.x; w < GPUDB_RS_WARPS * 256; w += GPUDB_RS_THREADS) cnt[w] = 0u;
+        __syncthreads();
+        const unsigned b = t * GPUDB_RS_TILE + warp * (GPUDB_RS_ITEMS * 32u) + lane;
+        unsigned long long k[GPUDB_RS_ITEMS];
+        unsigned x[GPUDB_RS_ITEMS], pos[GPUDB_RS_ITEMS];
+#pragma unroll
+        for (int u = 0; u < GPUDB_RS_ITEMS; ++u) {
+            const unsigned i = b + u * 32u;
+            k[u] = i < n ? __ldcg(kin + i) : 0ull;
+            x[u] = i < n ? __ldcg(xin + i) : 0u;
+        }
+#pragma unroll
+        for (int u = 0; u < GPUDB_RS_ITEMS; ++u) {
+            const bool in = b + u * 32u < n;
+            const unsigned d = in ? (unsigned)(k[u] >> shift) & 255u : 256u;
+            const unsigned peers = __match_any_sync(0xffffffffu, d);
+            const unsigned before = in ? cnt[warp * 256u + d] : 0u;
+            __syncwarp();
+            if (in && (int)lane == __ffs(peers) - 1) cnt[warp * 256u + d] = before + __popc(peers);
+            __syncwarp();
+            pos[u] = before + __popc(peers & ((1u << lane) - 1u));
+        }
+        __syncthreads();
+        if (threadIdx.x < 256u) {
+            unsigned at = base[threadIdx.x] + __ldcg(counts + threadIdx.x * ntiles + t);
+            for (int w = 0; w < GPUDB_RS_WARPS; ++w) {
+                const unsigned c = cnt[w * 256 + threadIdx.x];
+                cnt[w * 256 + threadIdx.x] = at;
+                at += c;
+            }
+        }
+        __syncthreads();
+#pragma unroll
+        for (int u = 0; u < GPUDB_RS_ITEMS; ++u) {
+            if (b + u * 32u >= n) continue;
+            const unsigned p = cnt[warp * 256u + ((unsigned)(k[u] >> shift) & 255u)] + pos[u];
+            kout[p] = k[u];
+            xout[p] = x[u];
+        }
+        __syncthreads();
+    }
+}
+
+// Sort by every digit in which the keys differ (`diff`: bits not equal in
+// all keys); *cur names the buffer set that holds the pairs. False when a
+// barrier gave up.
+__device__ __noinline__ bool gpudb_rs_sort(unsigned long long* k0, unsigned long long* k1, unsigned* x0, unsigned* x1,
+                                           unsigned n, unsigned long long diff, unsigned* counts, unsigned* totals,
+                                           unsigned* bar, unsigned& epoch, int* cur, unsigned* sh, unsigned* err) {
+    const unsigned ntiles = (n + GPUDB_RS_TILE - 1u) / GPUDB_RS_TILE;
+    for (int shift = 0; shift < 64; shift += 8) {
+        if (((diff >> shift) & 255ull) == 0ull) continue;
+        const int c = *cur;
+        gpudb_rs_count(c ? k1 : k0, n, shift, counts, ntiles, sh);
+        if (!gpudb_grid_barrier(bar, epoch, err)) return false;
+        gpudb_rs_scan(counts, ntiles, totals, sh);
+        if (!gpudb_grid_barrier(bar, epoch, err)) return false;
+        gpudb_rs_scatter(c ? k1 : k0, c ? x1 : x0, n, shift, counts, totals, ntiles, c ? k0 : k1,
+                         c ? x0 : x1, sh);
+        if (!gpudb_grid_barrier(bar, epoch, err)) return false;
+        *cur = c ^ 1;
+    }
+    return true;
 }
 
 // ------------------------------------------------------------------

@@ -706,14 +706,14 @@ CudaQueryPlan buildGroupBy(Spec& s, const TuneConfig& tune) {
 // ---- groupby_sorted: the skewed-key group-by with every group returned
 // in ORDER BY sum DESC, key ASC — the reference sorts such group rows on
 // the host (the Q18 post-processing, codegen_main.cpp:1105-1721); here the
-// created groups are compacted and merge-sorted on the GPU. The plan
-// carries merge passes for up to 2048 << 15 groups; passes beyond what the
-// run's group count needs return at once.
+// created groups are compacted and radix-sorted on the GPU, in as many
+// passes as the sums' differing digits need (`passes`, an upper bound that
+// an earlier plan shape took, is accepted and has no effect).
 CudaQueryPlan buildGroupBySorted(Spec& s, const TuneConfig& tune) {
     CudaQueryPlan plan;
     plan.name = "GROUPBY_SORTED";
     const std::string groupsExpr = s.str("groups", "zgroups");
-    const int passes = (int)s.num("passes", 15);
+    const long long passes = s.num("passes", 15);
     if (passes < 1 || passes > 20) throw std::runtime_error("groupby_sorted: passes must be in [1, 20]");
     {
         auto scan = makeScan(plan, "zprobe", {"z_key", "z_value"}, tune);
@@ -732,21 +732,12 @@ CudaQueryPlan buildGroupBySorted(Spec& s, const TuneConfig& tune) {
                                                   std::vector<std::string>{"count", "sum"}, "gsc", cap),
                 tune);
     TuneConfig st = tune;
-    st.blockSize = 512;
-    st.minBlocksPerSM = 1;
-    {
-        auto sp = std::make_unique<CudaSortPass>(CudaSortPass::Mode::Chunks, "gss", "gsc_n", cap);
-        sp->setInput("gsc_key", "gsc_count", "gsc_sum");
-        appendPhase(plan, "GS_sort_chunks", std::move(sp), st);
-    }
-    for (int p = 0; p < passes; p++)
-        appendPhase(plan, "GS_merge" + std::to_string(p),
-                    std::make_unique<CudaSortPass>(CudaSortPass::Mode::Merge, "gss", "gsc_n", cap, p), st);
-    {
-        auto sp = std::make_unique<CudaSortPass>(CudaSortPass::Mode::Emit, "gss", "gsc_n", cap);
-        sp->setOutputNames("key", "count", "sum");
-        appendPhase(plan, "GS_emit", std::move(sp), st);
-    }
+    st.blockSize = CudaGroupSort::kThreads;
+    st.minBlocksPerSM = 2;  // 64 registers: a second block per SM hides the scatter's latency
+    auto sort = std::make_unique<CudaGroupSort>("gss", "gsc_n", cap);
+    sort->setInput("gsc_key", "gsc_count", "gsc_sum");
+    sort->setOutputNames("key", "count", "sum");
+    appendPhase(plan, "GS_sort", std::move(sort), st);
     return plan;
 }
 
