@@ -134,6 +134,7 @@ _SIGNATURES = [
     # gpudb_engine.h
     ("gpudb_query_collect", C.c_int, [C.c_void_p, C.c_void_p, C.POINTER(C.c_void_p)]),
     ("gpudb_query_prepare", C.c_int, [C.c_void_p, C.c_char_p, C.c_char_p, C.POINTER(C.c_void_p)]),
+    ("gpudb_resident_tune", C.c_size_t, [C.c_char_p, C.c_uint64, C.c_char_p, C.c_size_t]),
     ("gpudb_query_free", None, [C.c_void_p]),
     ("gpudb_query_source", C.c_size_t, [C.c_void_p, C.c_char_p, C.c_size_t]),
     ("gpudb_query_describe", C.c_size_t, [C.c_void_p, C.c_char_p, C.c_size_t]),

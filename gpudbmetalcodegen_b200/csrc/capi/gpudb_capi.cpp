@@ -488,13 +488,25 @@ int gpudb_query_prepare(gpudb_ctx* ctx, const char* spec, const char* tune, gpud
     *out = nullptr;
     try {
         if (ctx) cudaSetDevice(ctx->qc->ex.device());
-        auto q = gpudb::prepareQuery(spec, tune ? tune : "", true, ctx != nullptr);
+        std::string t = tune ? tune : "";
+        if (ctx && t.empty())
+            t = gpudb::residentTune(spec, [&](const std::string& table) { return ctx->qc->ex.tableRows(table); });
+        auto q = gpudb::prepareQuery(spec, t, true, ctx != nullptr);
         *out = new gpudb_query{q};
         return GPUDB_OK;
     } catch (const std::exception& e) {
         const std::string m = e.what();
         const bool compile = m.find("NVRTC") != std::string::npos || m.find("cuModule") != std::string::npos;
         return fail(ctx, compile ? GPUDB_E_COMPILE : GPUDB_E_PLAN, m);
+    }
+}
+
+size_t gpudb_resident_tune(const char* spec, uint64_t rows, char* buf, size_t cap) {
+    if (!spec) return 0;
+    try {
+        return copyOut(gpudb::residentTune(spec, [&](const std::string&) { return (size_t)rows; }), buf, cap);
+    } catch (const std::exception&) {
+        return copyOut(std::string(), buf, cap);
     }
 }
 

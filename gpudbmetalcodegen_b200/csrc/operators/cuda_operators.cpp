@@ -37,19 +37,33 @@ KeyOps keyOps(const std::string& keyType, HashLayout layout, bool packedOk = fal
 
 bool isOne(const std::string& valueExpr) { return valueExpr == "1" || valueExpr == "1ll" || valueExpr == "1u"; }
 
-// Add `val` to sum j (of `slots` slots) of a shared-memory table whose sums
-// are (low, high) word pairs: low words at 2 j slots, high words at
-// (2 j + 1) slots. `unit`: val is 1 (a block sees fewer than 2^32 rows, so
-// the low word alone holds the count).
-std::string sharedAdd(const std::string& base, int j, int slots, const std::string& slot, const std::string& val, bool unit) {
-    const std::string lo = base + " + " + S(2ll * j * slots) + " + " + slot, hi = base + " + " + S((2ll * j + 1) * slots) + " + " + slot;
-    if (unit) return "gpudb_red_add_shared_u32(" + lo + ", 1u);";
-    return "gpudb_shared_add64(" + lo + ", " + hi + ", (unsigned long long)" + val + ");";
-}
-std::string sharedSum(const std::string& base, int j, int slots, const std::string& slot) {
-    return "(((unsigned long long)" + base + "[" + S((2ll * j + 1) * slots) + " + " + slot + "] << 32) | " + base + "[" +
-           S(2ll * j * slots) + " + " + slot + "])";
-}
+// The sums of a shared-memory table of `slots` slots: each an array of low
+// words followed by one of high words. A `unit` sum only ever adds 1 (a
+// block sees fewer than 2^32 rows), so its low words hold the count and it
+// has no others.
+struct SharedSums {
+    std::string base;
+    int slots;
+    std::vector<bool> unit;
+    int words() const {
+        int w = 0;
+        for (const bool u : unit) w += u ? slots : 2 * slots;
+        return w;
+    }
+    std::string at(int j, bool high, const std::string& slot) const {
+        long long w = high ? slots : 0;
+        for (int k = 0; k < j; k++) w += unit[k] ? slots : 2 * slots;
+        return base + " + " + S(w) + " + " + slot;
+    }
+    std::string add(int j, const std::string& slot, const std::string& val) const {
+        if (unit[j]) return "gpudb_red_add_shared_u32(" + at(j, false, slot) + ", 1u);";
+        return "gpudb_shared_add64(" + at(j, false, slot) + ", " + at(j, true, slot) + ", (unsigned long long)" + val + ");";
+    }
+    std::string sum(int j, const std::string& slot) const {
+        const std::string lo = "(unsigned long long)*(" + at(j, false, slot) + ")";
+        return unit[j] ? lo : "(((unsigned long long)*(" + at(j, true, slot) + ") << 32) | " + lo + ")";
+    }
+};
 
 // Bucket8 probes count buckets of 8 slots; keep the same slot budget.
 int probeArg(HashLayout layout, int maxProbe) {
@@ -998,6 +1012,7 @@ void CudaKeyedAgg::produce(CudaCodegen& cg, ConsumerFn consume) {
         });
     } else if (st == Strategy::Shared) {
         const int words = nb * vpb;
+        const SharedSums sums{"_ks", words, {false}};
         const int soff = cg.allocDynamicSmem(words * 8);
         cg.addComment("keyed aggregation: per-block shared-memory table of " + S(words) + " words, as (low, high) words");
         cg.addLine("unsigned* _ks = reinterpret_cast<unsigned*>(gpudb_smem + " + S(soff) + ");");
@@ -1010,10 +1025,10 @@ void CudaKeyedAgg::produce(CudaCodegen& cg, ConsumerFn consume) {
                     const auto& ag = aggregates_[j];
                     const std::string at = "_bucket * " + S(vpb) + " + " + S(ag.offset), v = "_kv" + S(j);
                     if (ag.isWide) {  // the two words of gpudb_acc128_add
-                        cg.addLine(sharedAdd("_ks", 0, words, at, "(" + v + " & 0xFFFFFFFFll)", false));
-                        cg.addLine(sharedAdd("_ks", 0, words, at + " + 1", "(" + v + " >> 32)", false));
+                        cg.addLine(sums.add(0, at, "(" + v + " & 0xFFFFFFFFll)"));
+                        cg.addLine(sums.add(0, at + " + 1", "(" + v + " >> 32)"));
                     } else {
-                        cg.addLine(sharedAdd("_ks", 0, words, at, v, isOne(ag.valueExpr)));
+                        cg.addLine(sums.add(0, at, v));
                     }
                 }
             }, " else { gpudb_set_error(gpudb_err, GPUDB_ERR_BOUNDS); }");
@@ -1021,7 +1036,7 @@ void CudaKeyedAgg::produce(CudaCodegen& cg, ConsumerFn consume) {
         });
         cg.addLine("__syncthreads();");
         cg.addBlock("for (int _w = threadIdx.x; _w < " + S(words) + "; _w += blockDim.x)", [&]() {
-            cg.addLine("const unsigned long long _v = " + sharedSum("_ks", 0, words, "_w") + ";");
+            cg.addLine("const unsigned long long _v = " + sums.sum(0, "_w") + ";");
             cg.addLine("if (_v != 0ull) atomicAdd(" + out + " + _w, _v);");
         });
     } else {
@@ -1084,14 +1099,16 @@ void CudaAtomicAgg::produce(CudaCodegen& cg, ConsumerFn consume) {
     cg.addBufferLengthParam(len, arrayName_);
     const int L = smemLog2_;
     const int slots = 1 << L;
+    SharedSums sums{"_ac_v", slots, {}};
+    for (const auto& a : arrs) sums.unit.push_back(!warpAgg_ && isOne(a.second));
     if (L > 0) {
         const int ko = cg.allocDynamicSmem(slots * 8);
-        const int vo = cg.allocDynamicSmem(slots * 8 * na);
+        const int vo = cg.allocDynamicSmem(sums.words() * 4);
         cg.addComment("per-block shared-memory cache of hot buckets (" + S(slots) + " slots)");
         cg.addLine("unsigned long long* _ac_k = reinterpret_cast<unsigned long long*>(gpudb_smem + " + S(ko) + ");");
         cg.addLine("unsigned* _ac_v = reinterpret_cast<unsigned*>(gpudb_smem + " + S(vo) + ");  // (low, high) words");
         cg.addLine("for (int _w = threadIdx.x; _w < " + S(slots) + "; _w += blockDim.x) _ac_k[_w] = GPUDB_EMPTY64;");
-        cg.addLine("for (int _w = threadIdx.x; _w < " + S(2 * slots * na) + "; _w += blockDim.x) _ac_v[_w] = 0u;");
+        cg.addLine("for (int _w = threadIdx.x; _w < " + S(sums.words()) + "; _w += blockDim.x) _ac_v[_w] = 0u;");
         cg.addLine("__syncthreads();");
     }
     child_->produce(cg, [&]() {
@@ -1106,8 +1123,7 @@ void CudaAtomicAgg::produce(CudaCodegen& cg, ConsumerFn consume) {
                 cg.addLine("const int _as = gpudb_smem_ht_slot64(_ac_k, " + S(L) + ", (unsigned long long)_ab, " +
                            S(smemProbe_) + ");");
                 cg.addBlock("if (_as >= 0)", [&]() {
-                    for (int j = 0; j < na; j++)
-                        cg.addLine(sharedAdd("_ac_v", j, slots, "_as", "_av" + S(j), !warpAgg_ && isOne(arrs[j].second)));
+                    for (int j = 0; j < na; j++) cg.addLine(sums.add(j, "_as", "_av" + S(j)));
                 }, " else {");
                 cg.increaseIndent();
                 for (int j = 0; j < na; j++)
@@ -1140,7 +1156,7 @@ void CudaAtomicAgg::produce(CudaCodegen& cg, ConsumerFn consume) {
             cg.addLine("if (_k == GPUDB_EMPTY64) continue;");
             for (int j = 0; j < na; j++) {
                 const std::string v = "_as" + S(j);
-                cg.addLine("const unsigned long long " + v + " = " + sharedSum("_ac_v", j, slots, "_w") + ";");
+                cg.addLine("const unsigned long long " + v + " = " + sums.sum(j, "_w") + ";");
                 cg.addLine("if (" + v + " != 0ull) atomicAdd(" + arrs[j].first + " + _k, " + v + ");");
             }
         });
@@ -1454,17 +1470,20 @@ void CudaHashGroupBy::produce(CudaCodegen& cg, ConsumerFn consume) {
     const int na = (int)aggs_.size();
     const int L = smemLog2_;
     const bool smem = L > 0 && ko.store == "unsigned long long";
+    // a count of rows that no warp aggregation has summed only ever adds 1
+    SharedSums sums{"_gs_v", 1 << L, {}};
+    for (const auto& a : aggs_) sums.unit.push_back(!warpAgg_ && isOne(a.valueExpr));
     if (smem) {
         const int slots = 1 << L;
         const int ko_off = cg.allocDynamicSmem(slots * 8);
-        const int vo_off = cg.allocDynamicSmem(slots * 8 * na);
+        const int vo_off = cg.allocDynamicSmem(sums.words() * 4);
         cg.addComment("per-block shared-memory pre-aggregation table (" + S(slots) +
                       " slots) for heavy hitters; sums as (low, high) words");
         cg.addLine("unsigned long long* _gs_k = reinterpret_cast<unsigned long long*>(gpudb_smem + " + S(ko_off) + ");");
         cg.addLine("unsigned* _gs_v = reinterpret_cast<unsigned*>(gpudb_smem + " + S(vo_off) + ");");
         cg.addBlock("for (int _w = threadIdx.x; _w < " + S(slots) + "; _w += blockDim.x)", [&]() {
             cg.addLine("_gs_k[_w] = GPUDB_EMPTY64;");
-            for (int j = 0; j < 2 * na; j++) cg.addLine("_gs_v[" + S(j * slots) + " + _w] = 0u;");
+            for (int w = 0; w < sums.words(); w += slots) cg.addLine("_gs_v[" + S(w) + " + _w] = 0u;");
         });
         cg.addLine("__syncthreads();");
     }
@@ -1515,8 +1534,6 @@ void CudaHashGroupBy::produce(CudaCodegen& cg, ConsumerFn consume) {
         cg.decreaseIndent();
         cg.addLine("}");
     };
-    // a count of rows that no warp aggregation has summed: always 1
-    auto unitAgg = [&](int j) { return !warpAgg_ && isOne(aggs_[j].valueExpr); };
     child_->produce(cg, [&]() {
         cg.addLine("const long long _gk = (long long)(" + keyExpr_ + ");");
         std::vector<std::string> vals;
@@ -1529,7 +1546,7 @@ void CudaHashGroupBy::produce(CudaCodegen& cg, ConsumerFn consume) {
                 cg.addLine("const int _gss = gpudb_smem_ht_slot64(_gs_k, " + S(L) + ", (unsigned long long)_gk, " +
                            S(smemProbe_) + ");");
                 cg.addBlock("if (_gss >= 0)", [&]() {
-                    for (int j = 0; j < na; j++) cg.addLine(sharedAdd("_gs_v", j, 1 << L, "_gss", "_gv" + S(j), unitAgg(j)));
+                    for (int j = 0; j < na; j++) cg.addLine(sums.add(j, "_gss", "_gv" + S(j)));
                 }, " else {");
                 cg.increaseIndent();
                 globalUpdate("(_gk)", vals);
@@ -1558,7 +1575,7 @@ void CudaHashGroupBy::produce(CudaCodegen& cg, ConsumerFn consume) {
             cg.addLine("const unsigned long long _fk = _gs_k[_w];");
             cg.addLine("if (_fk == GPUDB_EMPTY64) continue;");
             std::vector<std::string> vals;
-            for (int j = 0; j < na; j++) vals.push_back(sharedSum("_gs_v", j, 1 << L, "_w"));
+            for (int j = 0; j < na; j++) vals.push_back(sums.sum(j, "_w"));
             globalUpdate("(_fk)", vals);
         });
     }

@@ -175,6 +175,52 @@ TuneConfig TuneConfig::parse(const std::string& s) {
 }
 
 // ===================================================================
+// Tuning of a query prepared against resident tables when the caller names
+// none. Chosen by what a template's kernels are bound by (B200, times at the
+// sizes named: the generic defaults -> these):
+//   q1        thread-private accumulators in shared memory and a shallow ring
+//             with an L2 prefetch behind it, two CTAs per SM: 52 -> 10 us at
+//             60K rows, 96 -> 40 us at 6M, 484 -> 322 us at 60M.
+//   q6        streams: the deep ring with two rows per read from 2^25 rows on
+//             (236 -> 234 us at 60M; the prefetching form 240 us), a two-stage
+//             ring with prefetch below, where the start of the stream weighs
+//             (33 -> 27 us at 6M rows).
+//   lookups   (bitmap and map joins, the distinct count) wait for L2: a
+//             two-stage ring of smaller tiles leaves room for every thread
+//             slot of the SM, and staged rows are read four at a time where
+//             that measured no slower (60M rows: join_topk 283 -> 242 us,
+//             multi_join 825 -> 342, join_direct 533 -> 463, histogram
+//             1032 -> 779; 30M: mix_join 191 -> 123, distinct 117 -> 93).
+//   group-bys, hash join  no warp aggregation (equal keys of a warp meet in
+//             native shared-memory adds) and as large a shared table as
+//             leaves 2,048 threads per SM: 2^11 slots probed at most four
+//             times, 2^12 for the join's narrower ones. Rows into groups:
+//             120M Zipf(1.1) into 4.2M 3.60 -> 1.76 ms (2^10 slots 1.86, 2^12
+//             1.95); 30M uniform into 1M 897 -> 488 us; 10M into 1,000
+//             236 -> 72 us; 1M into 4,099 39 -> 19 us. Hash join of 30M rows
+//             with 2^20 keys, probe 566 -> 287 us.
+// ===================================================================
+std::string residentTune(const std::string& spec, const std::function<size_t(const std::string&)>& tableRows) {
+    const SpecMap m = parseSpec(spec);
+    const auto it = m.find("template");
+    const std::string t = it == m.end() ? "" : it->second;
+    if (t == "q1" || t == "scan_filter_groupagg") return "keyed=5;vec=2;bs=256;tile=448;stages=2;occ=2;l2pf=1";
+    if (t == "q6" || t == "scan_filter_sum") {
+        const size_t rows = tableRows ? tableRows("fact") : 0;
+        return rows && rows < (size_t(1) << 25) ? "stages=2;occ=2;tile=1024;l2pf=1" : "stages=4;vec=2";
+    }
+    if (t == "join_topk") return "stages=2;occ=4;warp=0;bvec=4;tkb=74";
+    if (t == "multi_join") return "stages=2;occ=4;tile=1920";
+    if (t == "join_direct" || t == "anti_join" || t == "histogram" || t == "mix_join" || t == "distinct")
+        return "stages=2;occ=4;tile=1920;vec=4";
+    if (t == "join_rows" || t == "q6_selvec" || t == "mix_agg") return "stages=2";
+    if (t == "groupby" || t == "groupby_sorted") return "warp=0;bs=1024;stages=2;smem=11;sprobe=4;occ=2;tile=992";
+    if (t == "mix_groupby" || t == "mix_topk") return "warp=0;stages=2;smem=11;sprobe=4;occ=2;tile=960";
+    if (t == "hashjoin") return "warp=0;bs=1024;stages=2;smem=12;occ=2;tile=1984";
+    return "";
+}
+
+// ===================================================================
 // Builders
 // ===================================================================
 namespace {
@@ -543,7 +589,6 @@ CudaQueryPlan buildAntiJoin(Spec& s, const TuneConfig& tune) {
         auto bin = std::make_unique<CudaComputeExpr>(std::move(anti), "_bin", "int", "(int)p_discount[i]");
         auto cnt = std::make_unique<CudaAtomicCount>(std::move(bin), "aj_count", "_bin", bins);
         auto sum = std::make_unique<CudaAtomicAgg>(std::move(cnt), "aj_sum", "_bin", "p_price[i]", bins);
-        sum->setWarpAggregate(true);
         sum->setSharedCache(4, 4);
         appendPhase(plan, "AJ_probe", std::move(sum), tune);
     }
@@ -665,7 +710,6 @@ CudaQueryPlan buildMultiJoin(Spec& s, const TuneConfig& tune) {
         auto same = std::make_unique<CudaSelection>(std::move(ls), "_cn == _sn");
         auto ag = std::make_unique<CudaAtomicAgg>(std::move(same), "mj_revenue", "_cn",
                                                   "l_price[i] * (100ll - l_discount[i])", "25");
-        ag->setWarpAggregate(true);
         ag->setSharedCache(5, 2);
         appendPhase(plan, "MJ_lines", std::move(ag), tune);
     }

@@ -146,6 +146,11 @@ struct TuneConfig {
     static TuneConfig parse(const std::string& s);  // "bs=512;scan=tma;tile=1024;stages=4;..."
 };
 
+// The tuning of a query over resident tables whose caller names none ("" =
+// the generic defaults); tableRows gives a registered table's rows, 0 if
+// unknown (or may be empty).
+std::string residentTune(const std::string& spec, const std::function<size_t(const std::string&)>& tableRows);
+
 using SpecMap = std::map<std::string, std::string>;
 SpecMap parseSpec(const std::string& spec);
 std::string canonicalSpec(const SpecMap& m);

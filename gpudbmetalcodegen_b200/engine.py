@@ -447,6 +447,12 @@ def templates() -> List[str]:
     return get_string(_lib.load().gpudb_list_templates).split(",")
 
 
+def resident_tune(spec: str, rows: int = 0) -> str:
+    """The tuning Context.prepare gives `spec` when the caller names none,
+    over tables of `rows` rows (0: unknown)."""
+    return get_string(_lib.load().gpudb_resident_tune, spec.encode(), rows)
+
+
 def colbin_inspect(path: str) -> dict:
     """Header and column directory of a .colbin v2 file (no GPU needed)."""
     lib = _lib.load()

@@ -33,6 +33,9 @@ typedef struct gpudb_result gpudb_result;
  * ctx == NULL the query is planned and compiled but not loaded (no GPU
  * needed). */
 int gpudb_query_prepare(gpudb_ctx* ctx, const char* spec, const char* tune, gpudb_query** out);
+/* The tuning gpudb_query_prepare gives a query of a context when the caller
+ * names none, for tables of `rows` rows (0: unknown). */
+size_t gpudb_resident_tune(const char* spec, uint64_t rows, char* buf, size_t cap);
 void gpudb_query_free(gpudb_query* q);
 /* The generated CUDA source (reference --dump-msl, codegen_main.cpp:343-380). */
 size_t gpudb_query_source(gpudb_query* q, char* buf, size_t cap);
