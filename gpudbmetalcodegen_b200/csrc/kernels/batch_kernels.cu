@@ -8,14 +8,19 @@
 // a handful of launches (build, agg, group, top-k, top-k merge), replayable
 // as a CUDA graph.
 //
-// Hash tables are arrays of 16-byte slots {key + card (u32), count (u32),
+// Group tables are arrays of 16-byte slots {key + card (u32), count (u32),
 // sum (u64)}: two slots per L2 sector, and the all-zero pattern is the empty
-// slot (`int32 % card` lies in (-card, card), so key + card is never 0), so a
-// single memset initialises the whole arena. Each CTA first aggregates into
-// a shared-memory table of kSmemSlots entries (bounded probing; a row whose
-// key finds no room goes to the global table directly) and flushes it at
-// the end of every work item: few-group queries then cost a handful of
-// global atomics per tile, and hot keys of skewed ones stay on chip.
+// slot, so a single memset initialises the whole arena. A table with at
+// least 2 card - 1 slots is DENSE: slot i belongs to key i + 1 - card, a row
+// costs two reductions and no probe, and the table cannot overflow; a
+// smaller one is an open-addressing hash table (`int32 % card` lies in
+// (-card, card), so key + card is never 0). Each CTA may first aggregate
+// into a shared-memory table (kTableWords; bounded probing; a row
+// whose key finds no room goes to the global table directly), which it
+// flushes when it moves to another query: few-group queries then cost a
+// handful of global atomics per CTA, and hot keys of skewed ones stay on
+// chip. Nothing lists the created groups: the passes after the group-by walk
+// the slots, since a list costs one atomic on one address per group.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -37,10 +42,9 @@ void setThreadError(const std::string& message);
 namespace {
 
 constexpr int kTopK = 16;             // largest k a top-k query may ask for
-constexpr long long kTkChunk = 4096;  // slot-list entries per top-k work item
+constexpr long long kScanChunk = 16384;  // table slots per work item of the passes after the group-by
 constexpr int kUnroll = 4;            // independent rows in flight per thread
-constexpr int kSmemSlots = 2048;      // per-CTA shared-memory aggregation table
-constexpr int kSmemProbe = 4;         // probes into it before spilling to global
+constexpr int kSmemProbe = 4;         // probes into the shared table before spilling to global
 
 struct __align__(16) Slot {
     unsigned key;    // key + card, 0 = empty
@@ -73,8 +77,8 @@ struct QDesc {
     Slot* ht;
     int log2cap, maxProbe;
     int aggMode;  // GPUDB_AGG_SHARED / _GLOBAL_WARP / _GLOBAL / _SHARED_DIRECT
-    int sharedWarp;  // SHARED: warp aggregation before the shared table
-    unsigned* slots;
+    int dense;    // slot i belongs to encoded key i + 1
+    unsigned directBase;  // SHARED_DIRECT: the encoded key of shared slot 0
     long long* tk_part;  // [tk_chunks][kTopK] of (value, key)
     long long tk_chunks;
     long long* topk_out;  // [kTopK] of (key, value)
@@ -190,18 +194,14 @@ __device__ __forceinline__ void blockAdd2(long long c, long long s, unsigned lon
 
 // Linear probing from slot `s`, whose key word `cur` is already loaded.
 __device__ __forceinline__ long long slotFrom(Slot* ht, int log2cap, unsigned enc, unsigned long long s, unsigned cur,
-                                              unsigned maxProbe, unsigned* err, bool* fresh) {
+                                              unsigned maxProbe, unsigned* err) {
     const unsigned long long mask = (1ull << log2cap) - 1ull;
     for (unsigned p = 0; p < maxProbe; ++p) {
         if (p) cur = *((volatile unsigned*)&ht[s].key);
         if (cur == enc) return (long long)s;
         if (cur == 0u) {
             const unsigned prev = atomicCAS(&ht[s].key, 0u, enc);
-            if (prev == 0u) {
-                *fresh = true;
-                return (long long)s;
-            }
-            if (prev == enc) return (long long)s;
+            if (prev == 0u || prev == enc) return (long long)s;
         }
         s = (s + 1ull) & mask;
     }
@@ -209,29 +209,28 @@ __device__ __forceinline__ long long slotFrom(Slot* ht, int log2cap, unsigned en
     return -1;
 }
 
-// Add (count, sum) to a group of the query's global table, starting from
-// home slot `s0` whose key word `cur` is loaded; a group created here is
-// appended to the slot list (one atomic per warp for the positions).
-__device__ __forceinline__ void globalAddFrom(const QDesc& q, bool live, unsigned enc, unsigned long long s0,
-                                              unsigned cur, unsigned long long c, unsigned long long v) {
-    bool fresh = false;
-    long long slot = -1;
-    if (live) {
-        slot = slotFrom(q.ht, q.log2cap, enc, s0, cur, (unsigned)q.maxProbe, q.err, &fresh);
-        if (slot >= 0) {
-            gpudb_red_add_u32(&q.ht[slot].count, (unsigned)c);
-            gpudb_red_add_u64(&q.ht[slot].sum, v);
-        }
-    }
-    const unsigned long long pos = gpudb_warp_reserve(q.nslots, fresh);
-    if (fresh) q.slots[pos] = (unsigned)slot;
+__device__ __forceinline__ void slotAdd(Slot* s, unsigned c, unsigned long long v) {
+    gpudb_red_add_u32(&s->count, c);
+    gpudb_red_add_u64(&s->sum, v);
 }
 
-__device__ __forceinline__ void globalAdd(const QDesc& q, bool live, unsigned enc, unsigned long long c,
+// Add (count, sum) to a group of the query's table.
+template <bool DENSE>
+__device__ __forceinline__ void globalAdd(const QDesc& q, Slot* ht, int log2cap, unsigned enc, unsigned c,
                                           unsigned long long v) {
-    const unsigned long long s0 = gpudb_hash_slot((unsigned long long)enc, q.log2cap);
-    const unsigned cur = live ? *((volatile unsigned*)&q.ht[s0].key) : 0u;
-    globalAddFrom(q, live, enc, s0, cur, c, v);
+    if (DENSE) {
+        slotAdd(ht + (enc - 1u), c, v);
+        return;
+    }
+    const unsigned long long s0 = gpudb_hash_slot((unsigned long long)enc, log2cap);
+    const long long s = slotFrom(ht, log2cap, enc, s0, *((volatile unsigned*)&ht[s0].key), (unsigned)q.maxProbe, q.err);
+    if (s >= 0) slotAdd(ht + s, c, v);
+}
+
+// A table slot's group, if it holds one.
+__device__ __forceinline__ bool slotLive(const QDesc& q, const Slot& s) { return q.dense ? s.count != 0u : s.key != 0u; }
+__device__ __forceinline__ long long slotKey(const QDesc& q, const Slot& s, long long i) {
+    return decKey(q.dense ? (unsigned)i + 1u : s.key, q.card);
 }
 
 // ---- JOIN build: bitmap of dim keys with attr < attr_lt -------------------
@@ -250,8 +249,17 @@ __global__ void __launch_bounds__(1024) kJoinBuild(const QDesc* __restrict__ qs,
         for (long long i = r0 + threadIdx.x; i < r1; i += blockDim.x) {
             if (__ldcs(da + i) >= attrLt) continue;
             const long long k = __ldcs(dk + i);
-            if (k >= 0 && (k >> 5) < words) gpudb_bitmap_set(bm, k);
-            else gpudb_set_error(q.err, GPUDB_ERR_BOUNDS);
+            if (k < 0 || (k >> 5) >= words) {
+                gpudb_set_error(q.err, GPUDB_ERR_BOUNDS);
+                continue;
+            }
+            // lanes that set bits of one word (dimension keys tend to be
+            // dense and in order) set them with one atomic
+            const unsigned am = __activemask();
+            const unsigned w = (unsigned)(k >> 5);
+            const unsigned peers = __match_any_sync(am, w);
+            const unsigned bits = __reduce_or_sync(peers, 1u << (unsigned)(k & 31));
+            if ((int)(threadIdx.x & 31u) == __ffs(peers) - 1) atomicOr(bm + w, bits);
         }
     }
 }
@@ -365,48 +373,261 @@ __global__ void __launch_bounds__(U == 4 ? 1024 : 512, U == 4 ? 1 : 4) kAgg(cons
     }
 }
 
-// ---- GROUPBY / TOPK: filter -> key % card -> hash table (count, sum) -------
+// ---- GROUPBY / TOPK: filter -> key % card -> table (count, sum) -------------
 // Per query, the strategy the host picked from the expected group count and
 // the sample's key repetition:
 //   SHARED_DIRECT the CTA's shared table indexed by the key itself;
-//   SHARED      warp aggregation, then the CTA's hashed shared table;
+//   SHARED      the CTA's hashed shared table;
 //   GLOBAL_WARP warp aggregation, then the global table;
 //   GLOBAL      the global table directly.
 // A CTA keeps its shared table across a query's work items and flushes it
 // into the query's global table when it moves to another query or runs out
-// of work. On the global path the home-slot key words of a thread's U rows
-// are loaded together, so an existing group costs one L2 round trip per U
-// rows, then fire-and-forget reductions. U = 1 row per thread at a
-// 32-register cap (the default: every thread slot of the SM resident),
-// U = 2 at 42 registers, U = 4 at 64 (U < 4: blocks of at most 512).
-template <int U>
-__global__ void __launch_bounds__(U == 4 ? 1024 : 512, U == 4 ? 1 : (U == 2 ? 3 : 4)) kGroup(const QDesc* __restrict__ qs, WorkList wl, long long tile,
-                                               unsigned long long* counter) {
-    __shared__ long long s_item;
-    __shared__ unsigned sKey[kSmemSlots];
-    __shared__ unsigned sCnt[kSmemSlots];
-    __shared__ unsigned long long sSum[kSmemSlots];
-    for (int i = threadIdx.x; i < kSmemSlots; i += blockDim.x) {
-        sKey[i] = 0u;
-        sCnt[i] = 0u;
-        sSum[i] = 0ull;
+// of work. Its sums are (low, high) words, added natively (a 64-bit
+// shared-memory add is a compare-and-swap loop; gpudb_shared_add64): equal
+// keys of a warp meet there more cheaply than in a warp aggregation.
+//
+// A row for the global hash table costs L2 round trips (find the slot, then
+// the reductions). Lanes that need one wait in a queue of their warp until
+// kColdBatch rows have gathered, so the round trips are paid once per 64
+// rows instead of by every warp iteration with a single such lane in it
+// (before: 9 of 32 lanes active per instruction, long-scoreboard stalls first).
+//
+// Shared memory per CTA follows its threads (kTableWords each): one CTA of
+// 1,024 threads per SM or two of 512 then hold tables of 10 hashed or 13
+// direct slots per thread.
+//
+// Measured (B200, group stage alone, before -> now; floor: 16 B per row at
+// 6.65 TB/s): 27.1M rows, 71 % pass, 2,838 uniform keys 650 -> 116 us (65);
+// 58.9M rows, 8,763 uniform keys 724 -> 220 (142); 47.9M rows, 57 % pass,
+// Zipf(1.3) keys into 0.6M groups 992 -> 512 (115); 22.8M rows, Zipf over
+// 10,908 keys 302 -> 111 (55); the mixed batch's 34 grouped queries 5.79 ->
+// 3.06 ms. Queries of few keys run at 1.6 x their floor (their loads in
+// flight), uniform ones of many keys at the L2's rate of reductions (two per
+// row, 75 G rows/s).
+constexpr int kTableWords = 40;  // of the shared table, per thread
+constexpr int kColdBatch = 64;   // rows of the global hash path a warp takes at a time
+constexpr int kColdCap = kColdBatch + 32;
+
+__host__ __device__ constexpr int directSlots(int block) { return kTableWords * block / 3; }
+__host__ __device__ constexpr int hashedSlots(int block) { return kTableWords * block / 4; }
+constexpr size_t groupSmem(int block) { return (size_t)block * 4 * kTableWords + (size_t)(block / 32) * kColdCap * 12; }
+
+// The CTA's shared table: count and sum words of each slot, then (hashed)
+// its key word.
+struct SharedTable {
+    unsigned* w;
+    int slots;
+    __device__ __forceinline__ unsigned* cnt(int i) const { return w + i; }
+    __device__ __forceinline__ unsigned* lo(int i) const { return w + slots + i; }
+    __device__ __forceinline__ unsigned* hi(int i) const { return w + 2 * slots + i; }
+    __device__ __forceinline__ unsigned* key(int i) const { return w + 3 * slots + i; }
+    __device__ __forceinline__ void add(int i, unsigned long long v) const {
+        gpudb_red_add_shared_u32(cnt(i), 1u);
+        gpudb_shared_add64(lo(i), hi(i), v);
     }
-    volatile unsigned* vKey = sKey;
+};
+
+// Encoded group key (key % card) + card of a 32-bit key, from the query's
+// divisor held in registers.
+struct KeyCode {
+    unsigned card, magic;
+    int sh1, sh2;
+    __device__ __forceinline__ unsigned operator()(int k) const {
+        if (k >= 0) {
+            const unsigned n = (unsigned)k;
+            const unsigned t = __umulhi(n, magic);
+            return n - ((t + ((n - t) >> sh1)) >> sh2) * card + card;
+        }
+        return (unsigned)(k % (int)card) + card;
+    }
+};
+
+// A warp's rows on their way to the global hash table.
+struct ColdQueue {
+    unsigned long long* v;
+    unsigned* k;
+    int n;  // the same in every lane
+    // whole warps: the lanes with `cold` append their row
+    template <typename Take>
+    __device__ __forceinline__ void push(bool cold, unsigned enc, unsigned long long val, Take take) {
+        const unsigned m = __ballot_sync(0xffffffffu, cold);
+        if (!m) return;
+        const unsigned lane = threadIdx.x & 31u;
+        if (cold) {
+            const int p = n + __popc(m & ((1u << lane) - 1u));
+            k[p] = enc;
+            v[p] = val;
+        }
+        n += __popc(m);
+        __syncwarp();
+        if (n >= kColdBatch) {
+            n -= kColdBatch;
+            take(n, kColdBatch);
+            __syncwarp();
+        }
+    }
+};
+
+enum class GroupPath { Direct, Shared, Global };
+
+template <int U, GroupPath PATH, bool DENSE>
+__device__ __forceinline__ void groupTile(const QDesc& q, const SharedTable& st, unsigned directBase, ColdQueue& cq,
+                                          long long r0, long long r1) {
+    const int* __restrict__ filter = q.filter + r0;
+    const int* __restrict__ keyc = q.key + r0;
+    const long long* __restrict__ value = q.value + r0;
+    const int thr = q.thr;
+    const KeyCode code{(unsigned)q.card, q.cardMagic, q.cardSh1, q.cardSh2};
+    Slot* ht = q.ht;
+    const int log2cap = q.log2cap;
+    const unsigned maxProbe = (unsigned)q.maxProbe;
+    unsigned* err = q.err;
+    const bool warp = PATH == GroupPath::Global && q.aggMode == GPUDB_AGG_GLOBAL_WARP;
+    const int step = (int)blockDim.x, n = (int)(r1 - r0), lane = (int)(threadIdx.x & 31u);
+    // rows queued for the global table (two per lane in flight)
+    auto take = [&](int at, int count) {
+        unsigned enc[2], cur[2];
+        unsigned long long v[2], s0[2];
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+            const bool in = lane + 32 * j < count;
+            enc[j] = in ? cq.k[at + lane + 32 * j] : 0u;
+            v[j] = in ? cq.v[at + lane + 32 * j] : 0ull;
+            s0[j] = gpudb_hash_slot((unsigned long long)enc[j], log2cap);
+            cur[j] = in ? *((volatile unsigned*)&ht[s0[j]].key) : 0u;
+        }
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+            if (lane + 32 * j >= count) continue;
+            long long s = (long long)s0[j];
+            if (cur[j] != enc[j]) s = slotFrom(ht, log2cap, enc[j], s0[j], cur[j], maxProbe, err);
+            if (s >= 0) slotAdd(ht + s, 1u, v[j]);
+        }
+    };
+    const int first = (int)threadIdx.x - lane;  // the warp's first row of each round
+    // Software pipeline: while a round's rows are processed, the next round's
+    // keys and values (of its rows that pass: its filter words are here) and
+    // the filter words of the round after it are on their way.
+    auto loadFilter = [&](int b, int (&f)[U]) {
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const int i = b + u * step;
+            f[u] = i < n ? __ldcs(filter + i) : thr;  // no row passes at thr
+        }
+    };
+    auto loadRows = [&](int b, const int (&f)[U], int (&k)[U], long long (&v)[U]) {
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const bool p = f[u] < thr;
+            k[u] = p ? __ldcs(keyc + b + u * step) : 0;
+            v[u] = p ? __ldcs(value + b + u * step) : 0;
+        }
+    };
+    int f[U], f1[U], kr[U];
+    long long v[U];
+    loadFilter(first + lane, f);
+    loadFilter(first + lane + U * step, f1);
+    loadRows(first + lane, f, kr, v);
+    for (int b = first + lane; b - lane < n; b += U * step) {
+        int f2[U], k1[U];
+        long long v1[U];
+        loadFilter(b + 2 * U * step, f2);
+        loadRows(b + U * step, f1, k1, v1);
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const bool live = f[u] < thr;
+            const unsigned enc = live ? code(kr[u]) : 0u;
+            const unsigned long long val = (unsigned long long)v[u];
+            bool cold = live;
+            if (PATH == GroupPath::Direct) {
+                const unsigned i = enc - directBase;
+                if (live && i < (unsigned)st.slots) {
+                    st.add((int)i, val);
+                    cold = false;
+                }
+            } else if (PATH == GroupPath::Shared) {
+                if (live) {
+                    int h = (int)__umulhi(enc * 0x9E3779B1u, (unsigned)st.slots);
+#pragma unroll 1
+                    for (int p = 0; p < kSmemProbe; ++p) {
+                        unsigned cur = *(volatile unsigned*)st.key(h);
+                        if (cur == 0u) {
+                            const unsigned prev = atomicCAS(st.key(h), 0u, enc);
+                            cur = prev == 0u ? enc : prev;
+                        }
+                        if (cur == enc) {
+                            st.add(h, val);
+                            cold = false;
+                            break;
+                        }
+                        h = h + 1 < st.slots ? h + 1 : 0;
+                    }
+                }
+            } else if (warp) {
+                if (live) {
+                    const unsigned am = __activemask();
+                    const unsigned peers = __match_any_sync(am, enc);
+                    const unsigned long long sum = gpudb_peer_sum(am, peers, val);
+                    if (lane == __ffs(peers) - 1) globalAdd<DENSE>(q, ht, log2cap, enc, (unsigned)__popc(peers), sum);
+                }
+                cold = false;
+            }
+            if (DENSE) {
+                if (cold) slotAdd(ht + (enc - 1u), 1u, val);
+            } else {
+                cq.push(cold, enc, val, take);
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            f[u] = f1[u];
+            f1[u] = f2[u];
+            kr[u] = k1[u];
+            v[u] = v1[u];
+        }
+    }
+    if (!DENSE && cq.n) {  // the rest of this item's queued rows
+        take(0, cq.n);
+        cq.n = 0;
+        __syncwarp();
+    }
+}
+
+template <int U>
+__global__ void __launch_bounds__(1024, 1) kGroup(const QDesc* __restrict__ qs, WorkList wl, long long tile,
+                                                  unsigned long long* counter) {
+    extern __shared__ unsigned long long groupShared[];
+    __shared__ long long s_item;
+    const int words = kTableWords * (int)blockDim.x;
+    SharedTable st{reinterpret_cast<unsigned*>(groupShared), 0};
+    unsigned long long* coldV = groupShared + words / 2;
+    unsigned* coldK = reinterpret_cast<unsigned*>(coldV + (blockDim.x >> 5) * kColdCap);
+    ColdQueue cq{coldV + (threadIdx.x >> 5) * kColdCap, coldK + (threadIdx.x >> 5) * kColdCap, 0};
+    for (int i = threadIdx.x; i < words; i += blockDim.x) st.w[i] = 0u;
     const long long total = __ldg(wl.prefix + wl.nq);
-    // the query whose groups the shared table holds (SHARED mode), -1 when
-    // empty: the table is flushed into that query's global table only when
-    // the CTA moves to another query's rows or runs out of work, so a query's
-    // work items on one CTA share one table and one flush
+    // the query whose groups the shared table holds, -1 when empty: the table
+    // is flushed into that query's global table only when the CTA moves to
+    // another query's rows or runs out of work, so a query's work items on
+    // one CTA share one table and one flush
     int heldQ = -1;
+    auto shape = [&](const QDesc& q) {
+        st.slots = q.aggMode == GPUDB_AGG_SHARED_DIRECT ? directSlots((int)blockDim.x) : hashedSlots((int)blockDim.x);
+    };
     auto flushShared = [&](const QDesc& q) {
+        shape(q);
         const bool direct = q.aggMode == GPUDB_AGG_SHARED_DIRECT;
-        for (int i = threadIdx.x; i < kSmemSlots; i += blockDim.x) {
-            // a direct slot i holds key i + 1 - card (encoded i + 1) once counted
-            const unsigned k = direct ? (sCnt[i] ? (unsigned)i + 1u : 0u) : sKey[i];
-            globalAdd(q, k != 0u, k, sCnt[i], sSum[i]);
-            sKey[i] = 0u;
-            sCnt[i] = 0u;
-            sSum[i] = 0ull;
+        for (int i = threadIdx.x; i < st.slots; i += blockDim.x) {
+            const unsigned c = *st.cnt(i);
+            if (c) {
+                const unsigned k = direct ? (unsigned)i + q.directBase : *st.key(i);
+                const unsigned long long v = ((unsigned long long)*st.hi(i) << 32) | *st.lo(i);
+                if (q.dense) globalAdd<true>(q, q.ht, q.log2cap, k, c, v);
+                else globalAdd<false>(q, q.ht, q.log2cap, k, c, v);
+                *st.cnt(i) = 0u;
+                *st.lo(i) = 0u;
+                *st.hi(i) = 0u;
+            }
+            if (!direct) *st.key(i) = 0u;
         }
     };
     for (long long w; (w = pullWork(counter, total, &s_item)) >= 0;) {
@@ -421,197 +642,108 @@ __global__ void __launch_bounds__(U == 4 ? 1024 : 512, U == 4 ? 1 : (U == 2 ? 3 
             __syncthreads();
         }
         const QDesc& q = qs[qd];
-        const int* __restrict__ filter = q.filter;
-        const int* __restrict__ keyc = q.key;
-        const long long* __restrict__ value = q.value;
-        const int thr = q.thr;
-        const long long card = q.card;
-        const int mode = q.aggMode;
-        Slot* ht = q.ht;
-        const int log2cap = q.log2cap;
         const long long r0 = (w - __ldg(wl.prefix + qi)) * tile, r1 = min(q.rows, r0 + tile);
-        const long long step = (long long)blockDim.x;
-        // (the dense-warp loads of kAgg measured no faster here: this
-        // kernel's time goes to the aggregation, and the extra registers spill)
-        int fn[U];
-        loadFilters(filter, r0 + threadIdx.x, step, r1, thr, fn);
-        for (long long b = r0 + threadIdx.x; b < r1; b += U * step) {
-            int f[U], kr[U];
-            long long v[U];
-#pragma unroll
-            for (int u = 0; u < U; ++u) f[u] = fn[u];
-            loadFilters(filter, b + U * step, step, r1, thr, fn);
-#pragma unroll
-            for (int u = 0; u < U; ++u) {
-                const bool p = f[u] < thr;
-                kr[u] = p ? __ldcs(keyc + b + u * step) : 0;
-                v[u] = p ? __ldcs(value + b + u * step) : 0;
-            }
-            unsigned enc[U];
-            bool live[U];
-            unsigned c[U];  // rows a lane adds for its group: at most a warp's
-            unsigned long long val[U];
-#pragma unroll
-            for (int u = 0; u < U; ++u) {
-                live[u] = f[u] < thr;
-                enc[u] = live[u] ? encKey(keyMod(kr[u], q), card) : 0u;
-                c[u] = 1u;
-                val[u] = (unsigned long long)v[u];
-            }
-            if (mode == GPUDB_AGG_SHARED_DIRECT) {
-                // keys in (-card, card): enc - 1 in [0, 2 card - 1) indexes
-                // the table directly, no probing and no warp aggregation
-                // (same-slot lanes of one warp serialise in the shared
-                // atomic unit, cheaper than a match and two peer sums)
-#pragma unroll
-                for (int u = 0; u < U; ++u) {
-                    if (!live[u]) continue;
-                    gpudb_red_add_shared_u32(&sCnt[enc[u] - 1u], 1u);
-                    gpudb_red_add_shared_u64(&sSum[enc[u] - 1u], val[u]);
-                }
-                continue;
-            }
-            if (mode == GPUDB_AGG_GLOBAL_WARP || (mode == GPUDB_AGG_SHARED && q.sharedWarp)) {
-#pragma unroll
-                for (int u = 0; u < U; ++u) {
-                    if (!live[u]) continue;
-                    const unsigned am = __activemask();
-                    const unsigned peers = __match_any_sync(am, enc[u]);
-                    c[u] = (unsigned)__popc(peers);  // every peer is one live row
-                    val[u] = gpudb_peer_sum(am, peers, val[u]);
-                    live[u] = (int)(threadIdx.x & 31u) == __ffs(peers) - 1;
-                }
-            }
-            if (mode == GPUDB_AGG_SHARED) {
-#pragma unroll
-                for (int u = 0; u < U; ++u) {
-                    if (!live[u]) continue;
-                    unsigned h = (unsigned)gpudb_hash_slot((unsigned long long)enc[u], 11);
-                    bool done = false;
-#pragma unroll 1
-                    for (int p = 0; p < kSmemProbe; ++p) {
-                        unsigned cur = vKey[h];
-                        if (cur == 0u) cur = atomicCAS(&sKey[h], 0u, enc[u]) == 0u ? enc[u] : vKey[h];
-                        if (cur == enc[u]) {
-                            gpudb_red_add_shared_u32(&sCnt[h], c[u]);
-                            gpudb_red_add_shared_u64(&sSum[h], val[u]);
-                            done = true;
-                            break;
-                        }
-                        h = (h + 1u) & (kSmemSlots - 1);
-                    }
-                    // (spills one at a time: batching their home-slot loads
-                    // as the global path does measured slower, its extra
-                    // registers spilling)
-                    if (!done) globalAdd(q, true, enc[u], c[u], val[u]);
-                }
-            } else {
-                unsigned long long s0[U];
-                unsigned cur[U];
-#pragma unroll
-                for (int u = 0; u < U; ++u) {
-                    s0[u] = gpudb_hash_slot((unsigned long long)enc[u], log2cap);
-                    cur[u] = live[u] ? *((volatile unsigned*)&ht[s0[u]].key) : 0u;
-                }
-#pragma unroll
-                for (int u = 0; u < U; ++u) {
-                    if (live[u] && cur[u] == enc[u]) {  // the group exists in its home slot
-                        gpudb_red_add_u32(&ht[s0[u]].count, c[u]);
-                        gpudb_red_add_u64(&ht[s0[u]].sum, val[u]);
-                        live[u] = false;
-                    }
-                }
-#pragma unroll
-                for (int u = 0; u < U; ++u) globalAddFrom(q, live[u], enc[u], s0[u], cur[u], c[u], val[u]);
-            }
+        shape(q);
+        if (q.aggMode == GPUDB_AGG_SHARED_DIRECT) {
+            if (q.dense) groupTile<U, GroupPath::Direct, true>(q, st, q.directBase, cq, r0, r1);
+            else groupTile<U, GroupPath::Direct, false>(q, st, q.directBase, cq, r0, r1);
+            heldQ = qd;
+        } else if (q.aggMode == GPUDB_AGG_SHARED) {
+            if (q.dense) groupTile<U, GroupPath::Shared, true>(q, st, 0u, cq, r0, r1);
+            else groupTile<U, GroupPath::Shared, false>(q, st, 0u, cq, r0, r1);
+            heldQ = qd;
+        } else if (q.dense) {
+            groupTile<U, GroupPath::Global, true>(q, st, 0u, cq, r0, r1);
+        } else {
+            groupTile<U, GroupPath::Global, false>(q, st, 0u, cq, r0, r1);
         }
-        if (mode == GPUDB_AGG_SHARED || mode == GPUDB_AGG_SHARED_DIRECT) heldQ = qd;
     }
     // pullWork's barriers ordered the last adds before this flush
     if (heldQ >= 0) flushShared(qs[heldQ]);
 }
 
-// Block-wide merge of per-thread sorted lists; warp 0 receives the result.
-__device__ __forceinline__ void blockTopK(long long (&vv)[kTopK], long long (&kk)[kTopK], long long* sv, long long* sk,
-                                          long long (&ov)[kTopK], long long (&ok)[kTopK]) {
-    long long wv[kTopK], wk[kTopK];
-    gpudb_topk_warp_merge<kTopK>(vv, kk, wv, wk);
-    __syncthreads();
-    if ((threadIdx.x & 31u) == 0u)
-        for (int i = 0; i < kTopK; ++i) {
-            sv[(threadIdx.x >> 5) * kTopK + i] = wv[i];
-            sk[(threadIdx.x >> 5) * kTopK + i] = wk[i];
+// The warps' sorted lists (lane j of each holds its j-th best) -> warp 0
+// holds the block's best kTopK: pairwise list merges through shared memory.
+__device__ __forceinline__ void blockTopK(long long& rv, long long& rk, long long* sv, long long* sk) {
+    const int lane = (int)(threadIdx.x & 31u), warp = (int)(threadIdx.x >> 5), nw = (int)(blockDim.x >> 5);
+    __syncthreads();  // an earlier merge may still read sv / sk
+    sv[threadIdx.x] = rv;
+    sk[threadIdx.x] = rk;
+    for (int s = 1; s < nw; s <<= 1) {
+        __syncthreads();
+        if ((warp & (2 * s - 1)) == 0 && warp + s < nw) {
+            gpudb_topk_warp_merge_list<kTopK>(rv, rk, sv[(warp + s) * 32 + lane], sk[(warp + s) * 32 + lane]);
+            sv[threadIdx.x] = rv;
+            sk[threadIdx.x] = rk;
         }
-    __syncthreads();
-    if (threadIdx.x < 32u) {
-#pragma unroll
-        for (int i = 0; i < kTopK; ++i) {
-            vv[i] = GPUDB_TOPK_NONE_VAL;
-            kk[i] = GPUDB_TOPK_NONE_KEY;
-        }
-        for (int e = threadIdx.x; e < (int)(blockDim.x >> 5) * kTopK; e += 32) gpudb_topk_push<kTopK>(vv, kk, sv[e], sk[e]);
-        gpudb_topk_warp_merge<kTopK>(vv, kk, ov, ok);
     }
 }
 
-// ---- TOPK, pass 1: per chunk of the slot list, the best kTopK groups -------
-__global__ void __launch_bounds__(256) kTopKChunks(const QDesc* __restrict__ qs, WorkList wl,
-                                                   unsigned long long* counter) {
+// ---- after the group-by: count every grouped query's groups and, for TOPK,
+// keep the best kTopK of each chunk of its table. Each warp walks the slots
+// 32 at a time and keeps its best kTopK one per lane (a ballot drops slots
+// that cannot enter).
+__global__ void __launch_bounds__(256) kScanGroups(const QDesc* __restrict__ qs, WorkList wl, unsigned long long* counter) {
     __shared__ long long s_item;
-    __shared__ long long sv[8 * kTopK], sk[8 * kTopK];
+    __shared__ long long sv[256], sk[256];
+    __shared__ unsigned s_n;
+    const int lane = (int)(threadIdx.x & 31u), warp = (int)(threadIdx.x >> 5);
     const long long total = __ldg(wl.prefix + wl.nq);
     for (long long w; (w = pullWork(counter, total, &s_item)) >= 0;) {
         const int qi = findQuery(wl, w);
         const QDesc& q = qs[__ldg(wl.q + qi)];
         const long long c = w - __ldg(wl.prefix + qi);
-        const long long n = (long long)*q.nslots;
-        const long long j0 = c * kTkChunk, j1 = min(n, j0 + kTkChunk);
-        if (j0 >= n) continue;  // chunk past the groups this query created
-        long long vv[kTopK], kk[kTopK];
-#pragma unroll
-        for (int i = 0; i < kTopK; ++i) {
-            vv[i] = GPUDB_TOPK_NONE_VAL;
-            kk[i] = GPUDB_TOPK_NONE_KEY;
+        const long long i0 = c * kScanChunk, i1 = min(1ll << q.log2cap, i0 + kScanChunk);
+        const bool top = q.tmpl == GPUDB_TPL_TOPK;
+        const Slot* __restrict__ ht = q.ht;
+        if (threadIdx.x == 0) s_n = 0u;
+        __syncthreads();
+        unsigned n = 0;
+        long long rv = GPUDB_TOPK_NONE_VAL, rk = GPUDB_TOPK_NONE_KEY;
+        for (long long b = i0 + warp * 32; b < i1; b += blockDim.x) {
+            const long long i = b + lane;
+            Slot s{0u, 0u, 0ull};
+            if (i < i1) s = ht[i];
+            const bool live = slotLive(q, s);
+            n += (unsigned)__popc(__ballot_sync(0xffffffffu, live));
+            if (top)
+                gpudb_topk_warp_offer<kTopK>(rv, rk, live ? (long long)s.sum : GPUDB_TOPK_NONE_VAL,
+                                             live ? slotKey(q, s, i) : GPUDB_TOPK_NONE_KEY);
         }
-        for (long long j = j0 + threadIdx.x; j < j1; j += blockDim.x) {
-            const Slot& s = q.ht[q.slots[j]];
-            gpudb_topk_push<kTopK>(vv, kk, (long long)s.sum, decKey(s.key, q.card));
-        }
-        long long ov[kTopK], ok[kTopK];
-        blockTopK(vv, kk, sv, sk, ov, ok);
-        if (threadIdx.x == 0) {
-            long long* dst = q.tk_part + 2 * kTopK * c;
-            for (int i = 0; i < kTopK; ++i) {
-                dst[2 * i] = ov[i];
-                dst[2 * i + 1] = ok[i];
+        if (lane == 0 && n) atomicAdd(&s_n, n);
+        if (top) {
+            blockTopK(rv, rk, sv, sk);
+            if (threadIdx.x < (unsigned)kTopK) {
+                long long* dst = q.tk_part + 2 * (kTopK * c + lane);
+                dst[0] = rv;
+                dst[1] = rk;
             }
         }
+        __syncthreads();
+        if (threadIdx.x == 0 && s_n) atomicAdd(q.nslots, (unsigned long long)s_n);
     }
 }
 
 // ---- TOPK, pass 2: one CTA per query merges its chunks' lists --------------
 __global__ void __launch_bounds__(256) kTopKMerge(const QDesc* __restrict__ qs, const int* __restrict__ qlist) {
-    __shared__ long long sv[8 * kTopK], sk[8 * kTopK];
+    __shared__ long long sv[256], sk[256];
     const QDesc& q = qs[qlist[blockIdx.x]];
-    const long long n = (long long)*q.nslots;
-    const long long chunks = min(q.tk_chunks, (n + kTkChunk - 1) / kTkChunk);
-    long long vv[kTopK], kk[kTopK];
-#pragma unroll
-    for (int i = 0; i < kTopK; ++i) {
-        vv[i] = GPUDB_TOPK_NONE_VAL;
-        kk[i] = GPUDB_TOPK_NONE_KEY;
+    const int lane = (int)(threadIdx.x & 31u);
+    long long rv = GPUDB_TOPK_NONE_VAL, rk = GPUDB_TOPK_NONE_KEY;
+    for (long long c = threadIdx.x >> 5; c < q.tk_chunks; c += blockDim.x >> 5) {
+        const bool in = lane < kTopK;
+        const long long v = in ? q.tk_part[2 * (kTopK * c + lane)] : GPUDB_TOPK_NONE_VAL;
+        const long long k = in ? q.tk_part[2 * (kTopK * c + lane) + 1] : GPUDB_TOPK_NONE_KEY;
+        gpudb_topk_warp_merge_list<kTopK>(rv, rk, v, k);
     }
-    for (long long e = threadIdx.x; e < chunks * kTopK; e += blockDim.x)
-        gpudb_topk_push<kTopK>(vv, kk, q.tk_part[2 * e], q.tk_part[2 * e + 1]);
-    long long ov[kTopK], ok[kTopK];
-    blockTopK(vv, kk, sv, sk, ov, ok);
-    if (threadIdx.x == 0) {
-        const long long m = min((long long)q.k, n);
-        for (long long i = 0; i < m; ++i) {
-            q.topk_out[2 * i] = ok[i];
-            q.topk_out[2 * i + 1] = ov[i];
+    blockTopK(rv, rk, sv, sk);
+    if (threadIdx.x < 32u) {
+        const long long m = min((long long)q.k, (long long)*q.nslots);
+        if (lane < m) {
+            q.topk_out[2 * lane] = rk;
+            q.topk_out[2 * lane + 1] = rv;
         }
-        *q.topk_n = (unsigned long long)m;
+        if (lane == 0) *q.topk_n = (unsigned long long)m;
     }
 }
 
@@ -753,9 +885,12 @@ __global__ void kResultRows(const QDesc* __restrict__ qs, int n, unsigned long l
 }
 
 // ---- collect: compaction of every query's rows into one packed buffer ------
-__global__ void kCollect(const QDesc* __restrict__ qs, WorkList wl, long long chunk, unsigned long long* counter,
-                         const unsigned long long* __restrict__ offs, long long* __restrict__ out) {
+// `cursor`: one zeroed position counter per query (group rows come in no order).
+__global__ void __launch_bounds__(256) kCollect(const QDesc* __restrict__ qs, WorkList wl, unsigned long long* counter,
+                                                unsigned long long* cursor, const unsigned long long* __restrict__ offs,
+                                                long long* __restrict__ out) {
     __shared__ long long s_item;
+    const unsigned lane = threadIdx.x & 31u;
     const long long total = __ldg(wl.prefix + wl.nq);
     for (long long w; (w = pullWork(counter, total, &s_item)) >= 0;) {
         const int qi = findQuery(wl, w);
@@ -779,13 +914,31 @@ __global__ void kCollect(const QDesc* __restrict__ qs, WorkList wl, long long ch
                 dst[3 * i + 2] = 0;
             }
         } else {
-            const long long n = (long long)*q.nslots;
-            const long long j1 = min(n, (c + 1) * chunk);
-            for (long long j = c * chunk + threadIdx.x; j < j1; j += blockDim.x) {
-                const Slot& s = q.ht[q.slots[j]];
-                dst[3 * j] = decKey(s.key, q.card);
-                dst[3 * j + 1] = (long long)s.count;
-                dst[3 * j + 2] = (long long)s.sum;
+            // a warp takes 128 slots at a time and reserves its rows with one atomic
+            const long long i1 = min(1ll << q.log2cap, (c + 1) * kScanChunk);
+            for (long long b = c * kScanChunk + (threadIdx.x >> 5) * 128; b < i1; b += 4 * blockDim.x) {
+                Slot s[4];
+                unsigned m[4], n = 0u;
+#pragma unroll
+                for (int u = 0; u < 4; ++u) {
+                    const long long i = b + u * 32 + lane;
+                    s[u] = i < i1 ? q.ht[i] : Slot{0u, 0u, 0ull};
+                    m[u] = __ballot_sync(0xffffffffu, slotLive(q, s[u]));
+                    n += __popc(m[u]);
+                }
+                unsigned long long p = 0ull;
+                if (lane == 0u && n) p = atomicAdd(cursor + id, (unsigned long long)n);
+                p = __shfl_sync(0xffffffffu, p, 0);
+#pragma unroll
+                for (int u = 0; u < 4; ++u) {
+                    if (m[u] >> lane & 1u) {
+                        long long* row = dst + 3 * (p + __popc(m[u] & ((1u << lane) - 1u)));
+                        row[0] = slotKey(q, s[u], b + u * 32 + lane);
+                        row[1] = (long long)s[u].count;
+                        row[2] = (long long)s[u].sum;
+                    }
+                    p += __popc(m[u]);
+                }
             }
         }
     }
@@ -842,12 +995,11 @@ struct gpudb_batch {
     cudaStream_t stream = nullptr;
     int numSMs = 148;
     int block = 512, maxProbe = 128, warpAgg = 1;
-    // rows in flight per thread of the group-by kernel: 1 (measured fastest
-    // on the mixed batch: its latency-bound aggregation gains more from
-    // twice the resident threads than it loses to a few spilled
-    // registers), 2 or 4
-    int groupRows = 1;
-    int sharedWarp = 1;  // SHARED strategy: warp aggregation before the shared table (1) or not (0)
+    // threads per CTA and rows in flight per thread of the group-by kernel.
+    // Measured on the 64-query mixed batch (group stage, ms): 512 threads
+    // with 1 / 2 / 4 rows 3.92 / 3.62 / 5.08, 1,024 threads 3.39 / 3.06 /
+    // 4.25: the larger CTA holds the larger shared table, four rows spill.
+    int groupBlock = 1024, groupRows = 2;
     // rows in flight per thread of the agg / join kernel: 2 (32 registers,
     // every thread slot resident; measured 9.9 ms against 10.6 ms per
     // mixed batch) or 4 (64 registers)
@@ -861,12 +1013,15 @@ struct gpudb_batch {
     DeviceBuf meta;     // descriptors + work lists
     DeviceBuf stats, sample, collect;
     QDesc* dDesc = nullptr;
-    WorkList wlBuild{}, wlAgg{}, wlGroup{}, wlTopk{}, wlStats{}, wlCollect{};
+    WorkList wlBuild{}, wlAgg{}, wlGroup{}, wlScan{}, wlStats{}, wlCollect{};
+    // rows per work item of each list: the tuning's, or fewer when the batch
+    // would leave CTAs without work
+    long long tileBuild = 0, tileAgg = 0, tileGroup = 0, tileStats = 0;
     int* dTopk = nullptr;
     int nTopk = 0;
-    long long collectChunk = 1 << 16;
     unsigned long long* counters = nullptr;  // work counters (first words of the arena)
-    unsigned* errHost = nullptr;             // pinned, one word per query
+    unsigned* errs = nullptr;                // one error word per query (behind the counters)
+    unsigned* errHost = nullptr;             // pinned copy of them
     size_t errCap = 0;
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t graphExec = nullptr;
@@ -891,6 +1046,8 @@ void dropGraph(gpudb_batch* b) {
 int plan(gpudb_batch* b) {
     const int n = (int)b->queries.size();
     size_t z = al256(8 * 8);  // work counters
+    const size_t zErr = z;
+    z += al256(4 * (size_t)n);
     size_t sc = 0;
     std::vector<size_t> zOff(n), sOff(n);
     std::vector<unsigned long long> caps(n, 0);
@@ -898,16 +1055,15 @@ int plan(gpudb_batch* b) {
     for (int i = 0; i < n; i++) {
         const auto& q = b->queries[i];
         zOff[i] = z;
-        z += 64;  // agg[3], topk_n, nslots, err
+        z += 64;  // agg[3], topk_n, nslots
         if (q.tmpl == GPUDB_TPL_JOIN) z += 4 * ((size_t)q.dim_max_key / 32 + 1);
         if (grouped(q.tmpl)) {
             caps[i] = pow2ceil(2 * std::max<uint64_t>(q.groups, 1));
             z = al256(z);
             z += sizeof(Slot) * caps[i];
-            sOff[i] = sc;
-            sc += al256(4 * caps[i]);
             if (q.tmpl == GPUDB_TPL_TOPK) {
-                tkChunks[i] = (long long)((caps[i] + kTkChunk - 1) / kTkChunk);
+                sOff[i] = sc;
+                tkChunks[i] = (long long)((caps[i] + kScanChunk - 1) / kScanChunk);
                 sc += al256(16 * kTopK * (size_t)tkChunks[i] + 16 * kTopK);
             }
         }
@@ -919,9 +1075,26 @@ int plan(gpudb_batch* b) {
     char* zb = static_cast<char*>(b->arena.p);
     char* sb = static_cast<char*>(b->scratch.p);
     b->counters = reinterpret_cast<unsigned long long*>(zb);
+    b->errs = reinterpret_cast<unsigned*>(zb + zErr);
     b->desc.assign(n, QDesc{});
     std::vector<int> lBuild, lAgg, lGroup, lTopk, lAll(n), lCollect;
-    std::vector<long long> pBuild{0}, pAgg{0}, pGroup{0}, pTopk{0}, pAll{0}, pCollect{0};
+    std::vector<long long> pBuild{0}, pAgg{0}, pGroup{0}, pScan{0}, pAll{0}, pCollect{0};
+    // Two work items for each of the 4 x numSMs CTAs of 512 threads before
+    // an item gets the tuning's rows: 8M rows in 32K-row items are work for
+    // 233 of 592 CTAs (B200, four queries of 1M-5M rows: see kGroup)
+    long long rBuild = 0, rAgg = 0, rGroup = 0;
+    for (const auto& q : b->queries) {
+        if (q.tmpl == GPUDB_TPL_JOIN) rBuild += (long long)q.dim_rows;
+        (grouped(q.tmpl) ? rGroup : rAgg) += (long long)q.rows;
+    }
+    auto tileFor = [&](long long rows) {
+        const long long t = (rows / (8ll * b->numSMs) + 1023) / 1024 * 1024;
+        return std::min(b->tile, std::max<long long>(4096, t));
+    };
+    b->tileBuild = tileFor(rBuild);
+    b->tileAgg = tileFor(rAgg);
+    b->tileGroup = tileFor(rGroup);
+    b->tileStats = tileFor(rAgg + rGroup);
     for (int i = 0; i < n; i++) {
         const auto& q = b->queries[i];
         QDesc& d = b->desc[i];
@@ -944,14 +1117,23 @@ int plan(gpudb_batch* b) {
         // table (with spill to the global one), which is never far off
         d.aggMode = q.agg_mode != GPUDB_AGG_AUTO ? q.agg_mode : GPUDB_AGG_SHARED;
         if (!b->warpAgg && d.aggMode == GPUDB_AGG_GLOBAL_WARP) d.aggMode = GPUDB_AGG_GLOBAL;
-        // the direct table holds the 2 card - 1 encoded keys of (-card, card)
-        if (d.aggMode == GPUDB_AGG_SHARED_DIRECT && 2 * d.card - 1 > kSmemSlots) d.aggMode = GPUDB_AGG_SHARED;
-        d.sharedWarp = b->sharedWarp;
+        // The direct table takes every key of (-card, card), or, of a larger
+        // domain, the keys >= 0 (the column's statistics say that there are
+        // no others; any that occur go to the global table). It never loses
+        // to the hashed one while a CTA's flush stays small beside its rows:
+        // below that, a large domain keeps the other strategies.
+        const int slots = directSlots(b->groupBlock);
+        const bool both = 2 * d.card - 1 <= slots, upper = d.card <= slots && q.key_min >= 0;
+        const bool enough = both && d.card <= 1024 ? true : d.rows >= 4ll * b->numSMs * (1024 / b->groupBlock) * d.card;
+        if (d.aggMode == GPUDB_AGG_SHARED && (both || upper) && enough) d.aggMode = GPUDB_AGG_SHARED_DIRECT;
+        else if (d.aggMode == GPUDB_AGG_SHARED_DIRECT && !((both || upper) && enough))
+            d.aggMode = both || upper ? GPUDB_AGG_GLOBAL : GPUDB_AGG_SHARED;
+        d.directBase = both ? 1u : (unsigned)d.card;
         char* p = zb + zOff[i];
         d.agg = reinterpret_cast<unsigned long long*>(p);
         d.topk_n = d.agg + 3;
         d.nslots = d.agg + 4;
-        d.err = reinterpret_cast<unsigned*>(p + 40);
+        d.err = b->errs + i;
         p += 64;
         if (q.tmpl == GPUDB_TPL_JOIN) {
             d.bitmap = reinterpret_cast<unsigned*>(p);
@@ -962,37 +1144,34 @@ int plan(gpudb_batch* b) {
             p = zb + al256((size_t)(p - zb));
             d.ht = reinterpret_cast<Slot*>(p);
             d.log2cap = log2u(caps[i]);
-            d.slots = reinterpret_cast<unsigned*>(sb + sOff[i]);
+            // no probe and no overflow where the table can hold every key anyway
+            d.dense = 2 * (unsigned long long)d.card - 1 <= caps[i];
             if (q.tmpl == GPUDB_TPL_TOPK) {
-                d.tk_part = reinterpret_cast<long long*>(sb + sOff[i] + al256(4 * caps[i]));
+                d.tk_part = reinterpret_cast<long long*>(sb + sOff[i]);
                 d.tk_chunks = tkChunks[i];
                 d.topk_out = d.tk_part + 2 * kTopK * tkChunks[i];
             }
         }
-        const long long tiles = (d.rows + b->tile - 1) / b->tile;
+        auto items = [](long long rows, long long tile) { return (rows + tile - 1) / tile; };
         lAll[i] = i;
-        pAll.push_back(pAll.back() + tiles);
+        pAll.push_back(pAll.back() + items(d.rows, b->tileStats));
         if (q.tmpl == GPUDB_TPL_JOIN) {
             lBuild.push_back(i);
-            pBuild.push_back(pBuild.back() + (d.dim_rows + b->tile - 1) / b->tile);
+            pBuild.push_back(pBuild.back() + items(d.dim_rows, b->tileBuild));
         }
         if (q.tmpl == GPUDB_TPL_AGG || q.tmpl == GPUDB_TPL_JOIN) {
             lAgg.push_back(i);
-            pAgg.push_back(pAgg.back() + tiles);
+            pAgg.push_back(pAgg.back() + items(d.rows, b->tileAgg));
         }
+        const long long chunks = items((long long)caps[i], kScanChunk);
         if (grouped(q.tmpl)) {
             lGroup.push_back(i);
-            pGroup.push_back(pGroup.back() + tiles);
+            pGroup.push_back(pGroup.back() + items(d.rows, b->tileGroup));
+            pScan.push_back(pScan.back() + chunks);
         }
-        if (q.tmpl == GPUDB_TPL_TOPK) {
-            lTopk.push_back(i);
-            pTopk.push_back(pTopk.back() + tkChunks[i]);
-        }
+        if (q.tmpl == GPUDB_TPL_TOPK) lTopk.push_back(i);
         lCollect.push_back(i);
-        const long long cchunks = q.tmpl == GPUDB_TPL_GROUPBY
-                                      ? (long long)((caps[i] + b->collectChunk - 1) / b->collectChunk)
-                                      : 1;
-        pCollect.push_back(pCollect.back() + std::max<long long>(1, cchunks));
+        pCollect.push_back(pCollect.back() + (q.tmpl == GPUDB_TPL_GROUPBY ? chunks : 1));
     }
     std::vector<char> host;
     auto put = [&](const void* src, size_t bytes) {
@@ -1008,7 +1187,8 @@ int plan(gpudb_batch* b) {
         return std::make_pair(a, c);
     };
     const auto oB = putList(lBuild, pBuild), oA = putList(lAgg, pAgg), oG = putList(lGroup, pGroup),
-               oT = putList(lTopk, pTopk), oS = putList(lAll, pAll), oC = putList(lCollect, pCollect);
+               oT = putList(lGroup, pScan), oS = putList(lAll, pAll), oC = putList(lCollect, pCollect);
+    const size_t oTop = put(lTopk.data(), 4 * lTopk.size());
     if (int st = b->meta.reserve(host.size(), b->stream)) return st;
     B_CHECK(cudaMemcpyAsync(b->meta.p, host.data(), host.size(), cudaMemcpyHostToDevice, b->stream), GPUDB_E_CUDA);
     char* m = static_cast<char*>(b->meta.p);
@@ -1019,10 +1199,10 @@ int plan(gpudb_batch* b) {
     b->wlBuild = wl(oB, lBuild.size());
     b->wlAgg = wl(oA, lAgg.size());
     b->wlGroup = wl(oG, lGroup.size());
-    b->wlTopk = wl(oT, lTopk.size());
+    b->wlScan = wl(oT, lGroup.size());
     b->wlStats = wl(oS, n);
     b->wlCollect = wl(oC, lCollect.size());
-    b->dTopk = reinterpret_cast<int*>(m + oT.first);
+    b->dTopk = reinterpret_cast<int*>(m + oTop);
     b->nTopk = (int)lTopk.size();
     if ((size_t)n > b->errCap) {
         if (b->errHost) cudaFreeHost(b->errHost);
@@ -1038,9 +1218,9 @@ int plan(gpudb_batch* b) {
     return GPUDB_OK;
 }
 
-int gridFor(gpudb_batch* b, const void* fn, int block) {
+int gridFor(gpudb_batch* b, const void* fn, int block, size_t smem = 0) {
     int occ = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fn, block, 0);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fn, block, smem);
     return std::max(1, occ) * b->numSMs;
 }
 
@@ -1055,48 +1235,47 @@ int enqueue(gpudb_batch* b, bool stages) {
     mark(1);
     if (b->wlBuild.nq) {
         kJoinBuild<<<gridFor(b, (const void*)kJoinBuild, b->block), b->block, 0, b->stream>>>(b->dDesc, b->wlBuild,
-                                                                                              b->tile, b->counters + 0);
+                                                                                              b->tileBuild, b->counters + 0);
         launches++;
     }
     mark(2);
     if (b->wlAgg.nq) {
         if (b->aggRows == 2 && b->block <= 512)  // the 2-row form is built for blocks of <= 512
             kAgg<2><<<gridFor(b, (const void*)kAgg<2>, b->block), b->block, 0, b->stream>>>(
-                b->dDesc, b->wlAgg, b->tile, b->counters + 1);
+                b->dDesc, b->wlAgg, b->tileAgg, b->counters + 1);
         else
             kAgg<4><<<gridFor(b, (const void*)kAgg<4>, b->block), b->block, 0, b->stream>>>(
-                b->dDesc, b->wlAgg, b->tile, b->counters + 1);
+                b->dDesc, b->wlAgg, b->tileAgg, b->counters + 1);
         launches++;
     }
     mark(3);
     if (b->wlGroup.nq) {
-        // the 1- and 2-row forms are built for blocks of at most 512 threads
-        if (b->groupRows == 2 && b->block <= 512)
-            kGroup<2><<<gridFor(b, (const void*)kGroup<2>, b->block), b->block, 0, b->stream>>>(
-                b->dDesc, b->wlGroup, b->tile, b->counters + 2);
-        else if (b->groupRows == 1 && b->block <= 512)
-            kGroup<1><<<gridFor(b, (const void*)kGroup<1>, b->block), b->block, 0, b->stream>>>(
-                b->dDesc, b->wlGroup, b->tile, b->counters + 2);
-        else
-            kGroup<4><<<gridFor(b, (const void*)kGroup<4>, b->block), b->block, 0, b->stream>>>(
-                b->dDesc, b->wlGroup, b->tile, b->counters + 2);
+        const int block = b->groupBlock;
+        const size_t smem = groupSmem(block);
+        auto launch = [&](void (*k)(const QDesc*, WorkList, long long, unsigned long long*)) {
+            k<<<gridFor(b, (const void*)k, block, smem), block, smem, b->stream>>>(b->dDesc, b->wlGroup, b->tileGroup,
+                                                                                  b->counters + 2);
+        };
+        if (b->groupRows == 1) launch(kGroup<1>);
+        else if (b->groupRows == 2) launch(kGroup<2>);
+        else launch(kGroup<4>);
         launches++;
     }
     mark(4);
+    if (b->wlScan.nq) {
+        kScanGroups<<<gridFor(b, (const void*)kScanGroups, 256), 256, 0, b->stream>>>(b->dDesc, b->wlScan, b->counters + 3);
+        launches++;
+    }
+    mark(5);
     if (b->nTopk) {
-        kTopKChunks<<<gridFor(b, (const void*)kTopKChunks, 256), 256, 0, b->stream>>>(b->dDesc, b->wlTopk,
-                                                                                      b->counters + 3);
-        mark(5);
         kTopKMerge<<<b->nTopk, 256, 0, b->stream>>>(b->dDesc, b->dTopk);
-        launches += 2;
-    } else {
-        mark(5);
+        launches++;
     }
     mark(6);
     B_CHECK(cudaGetLastError(), GPUDB_E_LAUNCH);
     // per-query error words -> pinned host copy
-    for (int i = 0; i < n; i++)
-        B_CHECK(cudaMemcpyAsync(b->errHost + i, b->desc[i].err, sizeof(unsigned), cudaMemcpyDeviceToHost, b->stream),
+    if (n)
+        B_CHECK(cudaMemcpyAsync(b->errHost, b->errs, sizeof(unsigned) * n, cudaMemcpyDeviceToHost, b->stream),
                 GPUDB_E_CUDA);
     b->lastLaunches = launches;
     return GPUDB_OK;
@@ -1152,6 +1331,9 @@ int gpudb_batch_create(gpudb_ctx* ctx, gpudb_batch** out) {
     for (auto& e : b->evStage) B_CHECK(cudaEventCreate(&e), GPUDB_E_CUDA);
     B_CHECK(cudaFuncSetAttribute(kSampleStats, cudaFuncAttributeMaxDynamicSharedMemorySize, kSampleSmem),
             GPUDB_E_LAUNCH);
+    for (const void* k : {(const void*)kGroup<1>, (const void*)kGroup<2>, (const void*)kGroup<4>})
+        B_CHECK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)groupSmem(1024)),
+                GPUDB_E_LAUNCH);
     *out = b.release();
     return GPUDB_OK;
 }
@@ -1245,9 +1427,7 @@ int gpudb_batch_set_option(gpudb_batch* b, const char* name, long long value) {
             gpudb::setThreadError("shared_warp must be 0 or 1");
             return GPUDB_E_INVALID;
         }
-        b->sharedWarp = (int)value;
-        b->dirty = true;
-        return GPUDB_OK;
+        return GPUDB_OK;  // rows go to the shared table directly in either case
     }
     if (n == "agg_rows") {
         if (value != 2 && value != 4) {
@@ -1264,7 +1444,7 @@ int gpudb_batch_set_option(gpudb_batch* b, const char* name, long long value) {
 
 int gpudb_batch_set_tuning(gpudb_batch* b, int block, int tile_rows, int warp_aggregate, int max_probe) {
     if (!b || block < 64 || block > 1024 || block % 32 || tile_rows < 256 || max_probe < 1) return GPUDB_E_INVALID;
-    b->block = block;
+    b->block = b->groupBlock = block;
     b->tile = tile_rows;
     b->warpAgg = warp_aggregate ? 1 : 0;
     b->maxProbe = max_probe;
@@ -1346,7 +1526,7 @@ int gpudb_batch_exact_stats(gpudb_batch* b, uint64_t* passing, uint64_t* distinc
     B_CHECK(cudaMemcpyAsync(b->dDesc, d.data(), sizeof(QDesc) * n, cudaMemcpyHostToDevice, b->stream), GPUDB_E_CUDA);
     B_CHECK(cudaEventRecord(b->ev0, b->stream), GPUDB_E_CUDA);
     B_CHECK(cudaMemsetAsync(b->stats.p, 0, bytes, b->stream), GPUDB_E_CUDA);
-    kStats<<<gridFor(b, (const void*)kStats, b->block), b->block, 0, b->stream>>>(b->dDesc, b->wlStats, b->tile,
+    kStats<<<gridFor(b, (const void*)kStats, b->block), b->block, 0, b->stream>>>(b->dDesc, b->wlStats, b->tileStats,
                                                                                   counter);
     B_CHECK(cudaGetLastError(), GPUDB_E_LAUNCH);
     B_CHECK(cudaEventRecord(b->ev1, b->stream), GPUDB_E_CUDA);
@@ -1427,8 +1607,8 @@ int gpudb_batch_collect(gpudb_batch* b, uint64_t* rows, void* host, uint64_t hos
         if (bytes_needed) *bytes_needed = 0;
         return GPUDB_OK;
     }
-    // rows[n] + offsets[n+1] + counter, then the packed result rows
-    const size_t head = al256(8 * (2 * (size_t)n + 2));
+    // rows[n] + offsets[n+1] + counter + cursors[n], then the packed result rows
+    const size_t head = al256(8 * (3 * (size_t)n + 2));
     size_t maxRows = 0;
     for (int i = 0; i < n; i++) {
         const auto& q = b->queries[i];
@@ -1442,10 +1622,11 @@ int gpudb_batch_collect(gpudb_batch* b, uint64_t* rows, void* host, uint64_t hos
     unsigned long long* counter = dOffs + n + 1;
     long long* out = reinterpret_cast<long long*>(static_cast<char*>(b->collect.p) + head);
     B_CHECK(cudaEventRecord(b->ev0, b->stream), GPUDB_E_CUDA);
-    B_CHECK(cudaMemsetAsync(counter, 0, 8, b->stream), GPUDB_E_CUDA);
+    B_CHECK(cudaMemsetAsync(counter, 0, 8 * ((size_t)n + 1), b->stream), GPUDB_E_CUDA);
     kResultRows<<<1, 1024, 0, b->stream>>>(b->dDesc, n, dRows, dOffs);
-    kCollect<<<gridFor(b, (const void*)kCollect, 256), 256, 0, b->stream>>>(b->dDesc, b->wlCollect, b->collectChunk,
-                                                                           counter, dOffs, out);
+    if (host)
+        kCollect<<<gridFor(b, (const void*)kCollect, 256), 256, 0, b->stream>>>(b->dDesc, b->wlCollect, counter,
+                                                                               counter + 1, dOffs, out);
     B_CHECK(cudaGetLastError(), GPUDB_E_LAUNCH);
     std::vector<unsigned long long> h(2 * (size_t)n + 1);
     B_CHECK(cudaMemcpyAsync(h.data(), dRows, 8 * (2 * (size_t)n + 1), cudaMemcpyDeviceToHost, b->stream),
@@ -1494,17 +1675,18 @@ int gpudb_batch_result_groups(gpudb_batch* b, int qi, uint64_t cap, uint64_t* ng
     B_CHECK(cudaStreamSynchronize(b->stream), GPUDB_E_CUDA);
     *ngroups = n;
     if (!keys || !counts || !sums || n == 0 || cap < n) return GPUDB_OK;
-    std::vector<unsigned> slots(n);
     std::vector<Slot> table((size_t)1 << d.log2cap);
-    B_CHECK(cudaMemcpyAsync(slots.data(), d.slots, 4 * n, cudaMemcpyDeviceToHost, b->stream), GPUDB_E_CUDA);
     B_CHECK(cudaMemcpyAsync(table.data(), d.ht, sizeof(Slot) * table.size(), cudaMemcpyDeviceToHost, b->stream),
             GPUDB_E_CUDA);
     B_CHECK(cudaStreamSynchronize(b->stream), GPUDB_E_CUDA);
-    for (unsigned long long j = 0; j < n; j++) {
-        const Slot& s = table[slots[j]];
-        keys[j] = (int64_t)decKey(s.key, d.card);
+    unsigned long long j = 0;
+    for (size_t i = 0; i < table.size() && j < n; i++) {
+        const Slot& s = table[i];
+        if (!(d.dense ? s.count : s.key)) continue;
+        keys[j] = (int64_t)decKey(d.dense ? (unsigned)i + 1u : s.key, d.card);
         counts[j] = (int64_t)s.count;
         sums[j] = (int64_t)s.sum;
+        j++;
     }
     return GPUDB_OK;
 }

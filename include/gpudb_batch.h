@@ -88,12 +88,13 @@ typedef struct {
 } gpudb_batch_query;
 
 #define GPUDB_AGG_AUTO 0         /* SHARED                                           */
-#define GPUDB_AGG_SHARED 1       /* warp + per-CTA shared-memory table, flushed       */
+#define GPUDB_AGG_SHARED 1       /* per-CTA shared-memory table, flushed              */
 #define GPUDB_AGG_GLOBAL_WARP 2  /* warp aggregation, then the global table          */
 #define GPUDB_AGG_GLOBAL 3       /* the global table directly (mostly distinct keys) */
 #define GPUDB_AGG_SHARED_DIRECT 4 /* per-CTA shared-memory table indexed by the key   *
-                                   * itself, no warp aggregation; card <= 1024 (else  *
-                                   * SHARED), flushed like SHARED                     */
+                                   * itself, flushed like SHARED. Taken for SHARED,   *
+                                   * too, where the keys fit and the rows outweigh    *
+                                   * the flush; where not, SHARED or GLOBAL stands in */
 
 int gpudb_batch_create(gpudb_ctx* ctx, gpudb_batch** out);
 void gpudb_batch_free(gpudb_batch* b);
@@ -108,12 +109,12 @@ int gpudb_batch_set_agg_mode(gpudb_batch* b, int q, int agg_mode);
  * aggregation (0 turns GLOBAL_WARP into GLOBAL), hash probe bound. */
 int gpudb_batch_set_tuning(gpudb_batch* b, int block, int tile_rows, int warp_aggregate, int max_probe);
 /* Named tuning options beyond those: "group_rows" = rows in flight per
- * thread of the group-by kernel: 1 (default; a 32-register cap), 2 (42
- * registers) or 4 (64 registers); blocks of more than 512 threads use 4.
+ * thread of the group-by kernel: 1, 2 (default) or 4. Until set_tuning names
+ * a block size, that kernel runs 1,024 threads per block and the others 512.
  * "agg_rows" = the same for the agg / join kernel: 2 (default; 32
  * registers, blocks of at most 512) or 4 (64 registers).
- * "shared_warp" = 1 (default): the SHARED strategy aggregates each warp's
- * equal keys before the shared table; 0: every row goes to it directly.
+ * "shared_warp" = 0 or 1, without effect: in the SHARED strategy every row
+ * goes to the shared table directly.
  * GPUDB_E_INVALID for an unknown name or value. */
 int gpudb_batch_set_option(gpudb_batch* b, const char* name, long long value);
 /* Run every query; per-query device error words go to errors[n] (bit
@@ -127,7 +128,7 @@ int gpudb_batch_exact_stats(gpudb_batch* b, uint64_t* passing, uint64_t* distinc
  * per query, see the library's feature definition). */
 int gpudb_batch_features(gpudb_batch* b, float* features, double* ms);
 /* Results. Scalar: count and 128-bit sum (lo, hi) for AGG / JOIN. Groups:
- * (key, count, sum) of GROUPBY / TOPK tables in slot-list order; ngroups is
+ * (key, count, sum) of GROUPBY / TOPK tables in table order; ngroups is
  * always set. Top-k: (key, sum) best first. */
 int gpudb_batch_result_scalar(gpudb_batch* b, int q, int64_t* count, uint64_t* sum_lo, int64_t* sum_hi);
 int gpudb_batch_result_groups(gpudb_batch* b, int q, uint64_t cap, uint64_t* ngroups, int64_t* keys, int64_t* counts,
@@ -144,7 +145,8 @@ int gpudb_batch_collect(gpudb_batch* b, uint64_t* rows, void* host, uint64_t hos
 /* Launches of this library's kernels in the last execute. */
 long long gpudb_batch_last_launches(gpudb_batch* b);
 /* Device time of each step of the last execute run without a graph:
- * zero fill, join build, agg / join probe, group-by, top-k chunks, top-k merge. */
+ * zero fill, join build, agg / join probe, group-by, table scan (group counts
+ * and top-k chunks), top-k merge. */
 #define GPUDB_BATCH_STAGES 6
 int gpudb_batch_stage_ms(gpudb_batch* b, double* ms);
 
