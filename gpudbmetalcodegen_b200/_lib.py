@@ -155,6 +155,7 @@ _SIGNATURES = [
     ("gpudb_result_export_i64", C.c_int, [C.c_void_p, C.c_int, C.c_void_p, C.c_longlong]),
     ("gpudb_result_canonical", C.c_size_t, [C.c_void_p, C.c_int, C.c_char_p, C.c_size_t]),
     ("gpudb_result_column_data", C.c_void_p, [C.c_void_p, C.c_int]),
+    ("gpudb_result_text", C.c_size_t, [C.c_void_p, C.c_char_p, C.c_size_t]),
     ("gpudb_result_free", None, [C.c_void_p]),
     ("gpudb_compare_canonical", C.c_int, [C.c_char_p, C.c_char_p, C.c_double, C.c_double, C.c_char_p,
                                           C.c_size_t]),

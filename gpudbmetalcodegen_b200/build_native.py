@@ -47,6 +47,7 @@ HOST_SOURCES = [
 CUDA_SOURCES: list[str] = [
     "kernels/noalloc_distinct.cu",
     "kernels/group_collect.cu",
+    "kernels/fill.cu",
     "kernels/sizer_mlp.cu",
     "kernels/batch_kernels.cu",
 ]

@@ -30,6 +30,17 @@ struct gpudb_query {
 };
 struct gpudb_result {
     gpudb::GenericResult r;
+    // serialised on first request: callers ask for the size, then the text
+    std::string text[2] = {};
+    bool serialised[2] = {false, false};
+    const std::string& canonical(int exact) {
+        const int e = exact ? 1 : 0;
+        if (!serialised[e]) {
+            text[e] = exact ? r.toExact() : r.toCanonical();
+            serialised[e] = true;
+        }
+        return text[e];
+    }
 };
 // An analyzed query under construction: its nodes are owned here and handed
 // out as opaque pointers (checked against this pool before use).
@@ -689,7 +700,30 @@ const int64_t* gpudb_result_column_data(gpudb_result* r, int col) {
 
 size_t gpudb_result_canonical(gpudb_result* r, int exact, char* buf, size_t cap) {
     if (!r) return 0;
-    return copyOut(exact ? r->r.toExact() : r->r.toCanonical(), buf, cap);
+    try {
+        return copyOut(r->canonical(exact), buf, cap);
+    } catch (const std::exception&) {
+        return 0;
+    }
+}
+
+size_t gpudb_result_text(gpudb_result* r, char* buf, size_t cap) {
+    if (!r) return 0;
+    try {
+        std::string types;
+        for (const auto& c : r->r.columns) types += c.type == "int" ? 'i' : c.type == "double" ? 'd' : 's';
+        const std::string* part[3] = {&types, &r->canonical(1), &r->canonical(0)};
+        size_t need = 0;
+        for (const auto* p : part) need += p->size() + 1;
+        if (buf && cap >= need)
+            for (const auto* p : part) {
+                std::memcpy(buf, p->c_str(), p->size() + 1);
+                buf += p->size() + 1;
+            }
+        return need;
+    } catch (const std::exception&) {
+        return 0;
+    }
 }
 
 void gpudb_result_free(gpudb_result* r) { delete r; }

@@ -45,7 +45,9 @@ CudaGenericExecutor::CudaGenericExecutor(int device) : device_(device) {
     GPUDB_CUDA_OR_THROW(cudaStreamCreateWithFlags(&stream_, cudaStreamNonBlocking));
     GPUDB_CUDA_OR_THROW(cudaMalloc((void**)&errWord_, sizeof(unsigned)));
     GPUDB_CUDA_OR_THROW(cudaMemset(errWord_, 0, sizeof(unsigned)));
-    GPUDB_CUDA_OR_THROW(cudaHostAlloc((void**)&errHost_, sizeof(unsigned), cudaHostAllocDefault));
+    // the error word's copy and the staging area share one pinned block
+    GPUDB_CUDA_OR_THROW(cudaHostAlloc((void**)&stageHost_, kStageBytes + 64, cudaHostAllocDefault));
+    errHost_ = reinterpret_cast<unsigned*>(stageHost_ + kStageBytes);
     const DriverApi& api = driverApi();
     if (!api.loaded) throw std::runtime_error("CUDA driver API unavailable: " + api.error);
 }
@@ -60,7 +62,7 @@ CudaGenericExecutor::~CudaGenericExecutor() {
     ownedColumns_.clear();
     for (auto e : events_) cudaEventDestroy(e);
     if (errWord_) cudaFree(errWord_);
-    if (errHost_) cudaFreeHost(errHost_);
+    if (stageHost_) cudaFreeHost(stageHost_);
     if (stream_) cudaStreamDestroy(stream_);
 }
 
@@ -311,7 +313,15 @@ GenericResult CudaGenericExecutor::collectResult(const CudaResultSchema& schema)
         if (collectGroupsOnDevice(schema, r)) return r;
     }
     return CudaResultCollector::collect(
-        schema, [this](const std::string& n, void* dst, size_t bytes) { return readBuffer(n, dst, bytes); },
+        schema,
+        [this](const std::string& n, void* dst, size_t bytes) {
+            for (const auto& s : staged_)
+                if (s.bytes == bytes && s.name == n) {
+                    std::memcpy(dst, stageHost_ + s.offset, bytes);
+                    return true;
+                }
+            return readBuffer(n, dst, bytes);
+        },
         [this](const std::string& e) { return resolver_.resolve(e); });
 }
 
@@ -366,12 +376,15 @@ bool CudaGenericExecutor::buildLaunch(const RuntimeCompiler::CompiledQuery& cq, 
             carveoutSet_[fkey] = ph.smemCarveout;
         }
     }
-    int occ = 0;
-    const CUresult r = api.cuOccupancyMaxActiveBlocksPerMultiprocessor(&occ, l.fn, (int)l.block, l.smem);
-    if (r != CUDA_SUCCESS || occ <= 0) {
-        error = "phase '" + ph.name + "' cannot be resident (block " + std::to_string(l.block) + ", smem " +
-                std::to_string(l.smem) + "): " + (r != CUDA_SUCCESS ? cuErrorString(r) : std::string("occupancy 0"));
-        return false;
+    int& occ = occupancy_[{cq.loadId, l.fn, l.block, l.smem}];
+    if (occ <= 0) {
+        const CUresult r = api.cuOccupancyMaxActiveBlocksPerMultiprocessor(&occ, l.fn, (int)l.block, l.smem);
+        if (r != CUDA_SUCCESS || occ <= 0) {
+            occ = 0;
+            error = "phase '" + ph.name + "' cannot be resident (block " + std::to_string(l.block) + ", smem " +
+                    std::to_string(l.smem) + "): " + (r != CUDA_SUCCESS ? cuErrorString(r) : std::string("occupancy 0"));
+            return false;
+        }
     }
     const long long maxRes = (long long)occ * numSMs_;
     long long grid = maxRes;
@@ -492,21 +505,21 @@ int CudaGenericExecutor::execute(const RuntimeCompiler::CompiledQuery& cq,
     for (int p = first; p < last; p++)
         if (!buildLaunch(cq, phases[p], launches[p - first], error)) return -4;
 
-    std::vector<Fill> fills;
+    std::vector<BufferFill> fills;
     if (!skipZeroInit_) {
-        std::map<void*, bool> seen;
+        std::unordered_set<void*> seen;
         for (int p = first; p < last; p++)
             for (const auto& b : phases[p].bindings) {
                 if (b.kind != CudaParamKind::DeviceBuffer || !b.zeroInit || b.readOnly) continue;
                 auto it = buffers_.find(b.name);
-                if (it == buffers_.end() || !it->second.ptr || seen[it->second.ptr]) continue;
-                seen[it->second.ptr] = true;
+                if (it == buffers_.end() || !it->second.ptr || !seen.insert(it->second.ptr).second) continue;
                 fills.push_back({it->second.ptr, it->second.bytes, b.fillByte});
             }
     }
 
     const size_t nl = launches.size();
-    ensureEvents(2 * nl + 2);
+    ensureEvents(nl + 1);
+    staged_.clear();
     out.phaseNames.clear();
     out.phaseTimesMs.assign(nl, 0.0);
     out.phaseGrid.clear();
@@ -521,18 +534,19 @@ int CudaGenericExecutor::execute(const RuntimeCompiler::CompiledQuery& cq,
     out.launches = (long long)nl;
     out.totalKernelTimeMs = 0.0;
 
+    // Timed iterations record an event after the fills and one after every
+    // kernel: a phase's time runs from the event before it to its own.
     auto launchAll = [&](bool timed) -> bool {
-        for (const auto& f : fills)
-            if (cudaMemsetAsync(f.ptr, f.value, f.bytes, stream_) != cudaSuccess) {
-                error = "cudaMemsetAsync failed";
-                return false;
-            }
-        if (timed) cudaEventRecord(events_[2 * nl], stream_);
+        if (fillBuffers(fills, stream_) != cudaSuccess) {
+            error = "buffer fill failed";
+            return false;
+        }
+        if (timed) cudaEventRecord(events_[0], stream_);
+        std::vector<void*> args;
         for (size_t i = 0; i < nl; i++) {
             Launch& l = launches[i];
-            std::vector<void*> args(l.slots.size());
+            args.resize(l.slots.size());
             for (size_t k = 0; k < l.slots.size(); k++) args[k] = &l.slots[k];
-            if (timed) cudaEventRecord(events_[2 * i], stream_);
             const CUresult r =
                 l.cooperative
                     ? api.cuLaunchCooperativeKernel(l.fn, l.grid, 1, 1, l.block, 1, 1, l.smem, (CUstream)stream_, args.data())
@@ -541,16 +555,24 @@ int CudaGenericExecutor::execute(const RuntimeCompiler::CompiledQuery& cq,
                 error = "launch of '" + l.name + "' failed: " + cuErrorString(r);
                 return false;
             }
-            if (timed) cudaEventRecord(events_[2 * i + 1], stream_);
+            if (timed) cudaEventRecord(events_[i + 1], stream_);
         }
-        if (timed) cudaEventRecord(events_[2 * nl + 1], stream_);
         return true;
     };
 
     // the word still holds the bits of deferred runs until they are read
-    if (!pendingErr_ && cudaMemsetAsync(errWord_, 0, sizeof(unsigned), stream_) != cudaSuccess) {
-        error = "cannot clear the device error word";
-        return -5;
+    if (!pendingErr_) {
+        if (useGraphs_) {
+            if (cudaMemsetAsync(errWord_, 0, sizeof(unsigned), stream_) != cudaSuccess) {
+                error = "cannot clear the device error word";
+                return -5;
+            }
+        } else if (warmup + measured == 1) {
+            fills.push_back({errWord_, sizeof(unsigned), 0});  // cleared by the run's own fills
+        } else if (cudaMemsetAsync(errWord_, 0, sizeof(unsigned), stream_) != cudaSuccess) {
+            error = "cannot clear the device error word";
+            return -5;
+        }
     }
     const int total = warmup + measured;
     std::map<std::string, GraphEntry>::iterator it = graphs_.end();
@@ -597,63 +619,84 @@ int CudaGenericExecutor::execute(const RuntimeCompiler::CompiledQuery& cq,
             graphOrder_.push_back(key);
         }
     }
-    if (it != graphs_.end()) {
-        for (int iter = 0; iter < total; iter++) {
-            const bool timed = iter >= warmup;
-            if (timed) cudaEventRecord(events_[2 * nl], stream_);
+    // The last iteration's wait also brings the error word and, after the
+    // plan's last phase, the small result buffers.
+    const bool stage = !defer && last == (int)phases.size();
+    unsigned bits = 0;
+    auto wait = [&](int iter, const char* what) -> bool {
+        cudaError_t e;
+        if (iter == total - 1) {
+            if (!stage) stageSchema_ = nullptr;
+            if (!enqueueTail()) {
+                error = "cannot read the device error word";
+                return false;
+            }
+            e = cudaStreamSynchronize(stream_);
+        } else {
+            e = cudaEventSynchronize(events_[nl]);
+        }
+        if (e != cudaSuccess) error = cudaErr(what, e);
+        return e == cudaSuccess;
+    };
+    const CudaResultSchema* const schema = stageSchema_;
+    for (int iter = 0; iter < total; iter++) {
+        const bool timed = iter >= warmup;
+        if (it != graphs_.end()) {
+            if (timed) cudaEventRecord(events_[0], stream_);
             if (cudaGraphLaunch(it->second.exec, stream_) != cudaSuccess) {
                 error = "cudaGraphLaunch failed";
                 return -6;
             }
-            if (timed) {
-                cudaEventRecord(events_[2 * nl + 1], stream_);
-                if (cudaEventSynchronize(events_[2 * nl + 1]) != cudaSuccess) {
-                    error = cudaErr("graph replay", cudaGetLastError());
-                    return -7;
-                }
-                float ms = 0;
-                cudaEventElapsedTime(&ms, events_[2 * nl], events_[2 * nl + 1]);
-                out.totalKernelTimeMs += ms / measured;
-            }
+            if (timed) cudaEventRecord(events_[nl], stream_);
+        } else if (!launchAll(timed)) {
+            return -6;
         }
-    } else {
-        for (int iter = 0; iter < total; iter++) {
-            const bool timed = iter >= warmup;
-            if (!launchAll(timed)) return -6;
-            if (timed) {
-                const cudaError_t e = cudaEventSynchronize(events_[2 * nl + 1]);
-                if (e != cudaSuccess) {
-                    error = cudaErr("kernel execution", e);
-                    return -7;
-                }
-                for (size_t i = 0; i < nl; i++) {
-                    float ms = 0;
-                    cudaEventElapsedTime(&ms, events_[2 * i], events_[2 * i + 1]);
-                    out.phaseTimesMs[i] += ms / measured;
-                }
-                float ms = 0;
-                cudaEventElapsedTime(&ms, events_[2 * nl], events_[2 * nl + 1]);
-                out.totalKernelTimeMs += ms / measured;
+        if (!timed) continue;
+        if (!wait(iter, it != graphs_.end() ? "graph replay" : "kernel execution")) return -7;
+        float ms = 0;
+        if (it == graphs_.end())
+            for (size_t i = 0; i < nl; i++) {
+                cudaEventElapsedTime(&ms, events_[i], events_[i + 1]);
+                out.phaseTimesMs[i] += ms / measured;
             }
-        }
+        cudaEventElapsedTime(&ms, events_[0], events_[nl]);
+        out.totalKernelTimeMs += ms / measured;
     }
     if (defer) {
         pendingErr_ = true;
         return 0;
     }
-    unsigned bits = 0;
-    if (!syncErrors(bits, error)) return -7;
+    stageSchema_ = stage ? nullptr : schema;  // a segment before the last leaves the request standing
+    if (!finishTail(bits, error)) return -7;
     out.deviceError |= bits;
     return 0;
 }
 
-bool CudaGenericExecutor::syncErrors(unsigned& bits, std::string& error) {
-    cudaError_t e = cudaMemcpyAsync(errHost_, errWord_, sizeof(unsigned), cudaMemcpyDeviceToHost, stream_);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(stream_);
-    if (e != cudaSuccess) {
-        error = cudaErr("kernel execution", e);
-        return false;
+void CudaGenericExecutor::stageResult(const CudaResultSchema* schema) {
+    stageSchema_ = schema;
+    staged_.clear();
+}
+
+// Enqueue the copies that follow a run's last kernel: the error word, and
+// the requested result buffers as far as they fit the staging area.
+bool CudaGenericExecutor::enqueueTail() {
+    if (stageSchema_) {
+        size_t at = 0;
+        for (const auto& [name, bytes] : CudaResultCollector::smallReads(
+                 *stageSchema_, [this](const std::string& e) { return resolver_.resolve(e); }, kStageBytes)) {
+            auto b = buffers_.find(name);
+            if (b == buffers_.end() || !b->second.ptr || bytes > b->second.bytes || at + bytes > kStageBytes) continue;
+            if (cudaMemcpyAsync(stageHost_ + at, b->second.ptr, bytes, cudaMemcpyDeviceToHost, stream_) != cudaSuccess)
+                return false;
+            staged_.push_back({name, bytes, at});
+            at += (bytes + 15) & ~size_t(15);
+        }
     }
+    return cudaMemcpyAsync(errHost_, errWord_, sizeof(unsigned), cudaMemcpyDeviceToHost, stream_) == cudaSuccess;
+}
+
+// The error bits that enqueueTail() brought (the stream has been waited for).
+bool CudaGenericExecutor::finishTail(unsigned& bits, std::string& error) {
     bits = *errHost_;
     if (pendingErr_) {
         // read: the next run starts from a clear word
@@ -664,6 +707,16 @@ bool CudaGenericExecutor::syncErrors(unsigned& bits, std::string& error) {
         }
     }
     return true;
+}
+
+bool CudaGenericExecutor::syncErrors(unsigned& bits, std::string& error) {
+    cudaError_t e = cudaMemcpyAsync(errHost_, errWord_, sizeof(unsigned), cudaMemcpyDeviceToHost, stream_);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(stream_);
+    if (e != cudaSuccess) {
+        error = cudaErr("kernel execution", e);
+        return false;
+    }
+    return finishTail(bits, error);
 }
 
 }  // namespace gpudb

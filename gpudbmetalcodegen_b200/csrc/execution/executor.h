@@ -9,8 +9,9 @@
 // zero/0xFF-fill them every iteration (unless skip-zero-init), launch the
 // phases in order, time them, and hand buffers to the collector.
 // B200 design:
-//   * one CUDA stream per executor; all fills and launches are
-//     stream-ordered, the host synchronises once per execute();
+//   * one CUDA stream per executor; all fills (one launch) and kernels are
+//     stream-ordered, the host synchronises once per execute(), and the
+//     error word and a small result come back under that same wait;
 //   * per-phase CUDA events (the reference's GPU timestamps);
 //   * launch = min(work, SMs x occupancy) persistent CTAs, with the
 //     dynamic shared memory each phase declares (TMA ring, smem tables);
@@ -23,11 +24,13 @@
 #include <map>
 #include <memory>
 #include <string>
+#include <tuple>
 #include <unordered_map>
 #include <unordered_set>
 #include <vector>
 
 #include "../core/cuda_codegen.h"
+#include "fill.h"
 #include "group_collect.h"
 #include "result_collector.h"
 #include "runtime_compiler.h"
@@ -107,6 +110,10 @@ public:
     void* bufferPtr(const std::string& name, size_t* bytes = nullptr) const;
     void releaseAllocatedBuffers();
     GenericResult collectResult(const CudaResultSchema& schema);
+    // The next execute() that reaches the plan's last phase also copies the
+    // small buffers `schema` is decoded from, so that collectResult() after
+    // it finds them on the host. nullptr drops what was staged.
+    void stageResult(const CudaResultSchema* schema);
     bool collectGroupsOnDevice(const CudaResultSchema& schema, GenericResult& r);
 
     cudaStream_t stream() const { return stream_; }
@@ -141,11 +148,6 @@ private:
         std::vector<uint64_t> slots;
         std::string name;
     };
-    struct Fill {
-        void* ptr;
-        size_t bytes;
-        int value;
-    };
 
     int device_ = 0;
     int numSMs_ = 148;
@@ -167,7 +169,20 @@ private:
     // keyed by (load id, function): handles of an unloaded module recur
     std::map<std::pair<uint64_t, CUfunction>, int> smemConfigured_;
     std::map<std::pair<uint64_t, CUfunction>, int> carveoutSet_;
+    // blocks per SM of (load id, function, block, dynamic shared memory)
+    std::map<std::tuple<uint64_t, CUfunction, unsigned, unsigned>, int> occupancy_;
     std::vector<cudaEvent_t> events_;
+    // pinned copies of the buffers a result is decoded from
+    struct Staged {
+        std::string name;
+        size_t bytes, offset;
+    };
+    static constexpr size_t kStageBytes = 64 * 1024;
+    char* stageHost_ = nullptr;
+    const CudaResultSchema* stageSchema_ = nullptr;
+    std::vector<Staged> staged_;
+    bool enqueueTail();
+    bool finishTail(unsigned& bits, std::string& error);
     GroupWorkspace groupScratch_;  // device scratch of group collection, grown on demand
     struct GraphEntry {
         cudaGraph_t graph = nullptr;

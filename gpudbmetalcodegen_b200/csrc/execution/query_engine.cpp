@@ -220,6 +220,13 @@ int runPhases(QueryContext& qc, PreparedQuery& q, const std::vector<int>& cuts, 
     return 0;
 }
 
+// What a run stages for its result is good until the call returns.
+struct StagedResult {
+    CudaGenericExecutor& ex;
+    StagedResult(CudaGenericExecutor& e, const CudaResultSchema* schema) : ex(e) { ex.stageResult(schema); }
+    ~StagedResult() { ex.stageResult(nullptr); }
+};
+
 int finish(QueryContext& qc, PreparedQuery& q, bool collect, ExecutionResult& out, std::string& err) {
     if (out.deviceError) {
         char b[16];
@@ -256,6 +263,7 @@ int runQuery(QueryContext& qc, PreparedQuery& q, int warmup, int measured, bool 
     out.codegenTimeMs = q.codegenMs;
     out.compileTimeMs = q.compileMs;
     size_t si = 0;
+    StagedResult staged(qc.ex, collect ? &q.cg.getResultSchema() : nullptr);
     if (int rc = runPhases(qc, q, cuts, 0, (int)phases.size(), warmup, measured, si, out, err)) return rc;
     return finish(qc, q, collect, out, err);
 }

@@ -173,6 +173,34 @@ GenericResult CudaResultCollector::collect(const CudaResultSchema& s, const Buff
     }
 }
 
+std::vector<std::pair<std::string, size_t>> CudaResultCollector::smallReads(const CudaResultSchema& s,
+                                                                            const SizeEval& size, size_t limit) {
+    std::vector<std::pair<std::string, size_t>> r;
+    auto add = [&](const std::string& name, size_t bytes) {
+        if (bytes && bytes <= limit) r.emplace_back(name, bytes);
+    };
+    switch (s.kind) {
+        case CudaResultSchema::SCALAR_AGG:
+            for (const auto& e : s.scalarAggs) add(e.buffer, e.isWide ? 16 : 8);
+            break;
+        case CudaResultSchema::KEYED_AGG:
+            add(s.keyedAgg.bufferName, (size_t)s.keyedAgg.numBuckets * s.keyedAgg.valuesPerBucket * 8);
+            break;
+        case CudaResultSchema::TOPK:
+            add(s.topk.countBuffer, 8);
+            add(s.topk.keyBuffer, 8 * (size_t)s.topk.k);
+            add(s.topk.valueBuffer, 8 * (size_t)s.topk.k);
+            for (const auto& e : s.topk.extra) add(e.buffer, (size_t)s.topk.k * cudaTypeBytes(e.elementType));
+            break;
+        case CudaResultSchema::DIRECT_AGG:
+            for (const auto& a : s.directAgg.aggs) add(a.buffer, (size_t)size(s.directAgg.sizeExpr) * 8);
+            break;
+        case CudaResultSchema::MATERIALIZE: add(s.counterBuffer, 8); break;
+        default: break;
+    }
+    return r;
+}
+
 GenericResult CudaResultCollector::collectScalarAgg(const CudaResultSchema& s, const BufferReader& read) {
     GenericResult r;
     GenericResult::Row row;

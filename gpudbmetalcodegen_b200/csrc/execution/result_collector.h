@@ -16,6 +16,7 @@
 #include <functional>
 #include <memory>
 #include <string>
+#include <utility>
 #include <variant>
 #include <vector>
 
@@ -69,6 +70,10 @@ using SizeEval = std::function<uint64_t(const std::string& expr)>;
 class CudaResultCollector {
 public:
     static GenericResult collect(const CudaResultSchema& schema, const BufferReader& read, const SizeEval& size);
+    // The reads of collect() that need no earlier one's answer, each of at
+    // most `limit` bytes (they can be issued before the run is waited for).
+    static std::vector<std::pair<std::string, size_t>> smallReads(const CudaResultSchema& schema, const SizeEval& size,
+                                                                  size_t limit);
 
 private:
     static GenericResult collectScalarAgg(const CudaResultSchema& s, const BufferReader& read);

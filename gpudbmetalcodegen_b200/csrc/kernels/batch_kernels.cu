@@ -1026,6 +1026,9 @@ struct gpudb_batch {
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t graphExec = nullptr;
     bool dirty = true;
+    // rows per query, their offsets and total of the last execution, once a
+    // collect has asked for them (their device copies stay in `collect`)
+    std::vector<unsigned long long> resultRows;
     long long lastLaunches = 0;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     cudaEvent_t evStage[GPUDB_BATCH_STAGES + 1] = {};
@@ -1214,6 +1217,7 @@ int plan(gpudb_batch* b) {
     }
     B_CHECK(cudaStreamSynchronize(b->stream), GPUDB_E_CUDA);
     dropGraph(b);
+    b->resultRows.clear();
     b->dirty = false;
     return GPUDB_OK;
 }
@@ -1458,6 +1462,7 @@ int gpudb_batch_execute(gpudb_batch* b, int use_graph, double* ms, uint32_t* err
     if (b->dirty)
         if (int st = plan(b)) return st;
     const int n = (int)b->queries.size();
+    b->resultRows.clear();
     B_CHECK(cudaEventRecord(b->ev0, b->stream), GPUDB_E_CUDA);
     if (use_graph) {
         if (!b->graphExec) {
@@ -1622,16 +1627,15 @@ int gpudb_batch_collect(gpudb_batch* b, uint64_t* rows, void* host, uint64_t hos
     unsigned long long* counter = dOffs + n + 1;
     long long* out = reinterpret_cast<long long*>(static_cast<char*>(b->collect.p) + head);
     B_CHECK(cudaEventRecord(b->ev0, b->stream), GPUDB_E_CUDA);
-    B_CHECK(cudaMemsetAsync(counter, 0, 8 * ((size_t)n + 1), b->stream), GPUDB_E_CUDA);
-    kResultRows<<<1, 1024, 0, b->stream>>>(b->dDesc, n, dRows, dOffs);
-    if (host)
-        kCollect<<<gridFor(b, (const void*)kCollect, 256), 256, 0, b->stream>>>(b->dDesc, b->wlCollect, counter,
-                                                                               counter + 1, dOffs, out);
-    B_CHECK(cudaGetLastError(), GPUDB_E_LAUNCH);
-    std::vector<unsigned long long> h(2 * (size_t)n + 1);
-    B_CHECK(cudaMemcpyAsync(h.data(), dRows, 8 * (2 * (size_t)n + 1), cudaMemcpyDeviceToHost, b->stream),
-            GPUDB_E_CUDA);
-    B_CHECK(cudaStreamSynchronize(b->stream), GPUDB_E_CUDA);
+    std::vector<unsigned long long>& h = b->resultRows;
+    if (h.empty()) {
+        kResultRows<<<1, 1024, 0, b->stream>>>(b->dDesc, n, dRows, dOffs);
+        B_CHECK(cudaGetLastError(), GPUDB_E_LAUNCH);
+        std::vector<unsigned long long> got(2 * (size_t)n + 1);
+        B_CHECK(cudaMemcpyAsync(got.data(), dRows, 8 * got.size(), cudaMemcpyDeviceToHost, b->stream), GPUDB_E_CUDA);
+        B_CHECK(cudaStreamSynchronize(b->stream), GPUDB_E_CUDA);
+        h = std::move(got);
+    }
     const unsigned long long total = h[2 * (size_t)n];
     if (rows)
         for (int i = 0; i < n; i++) rows[i] = h[i];
@@ -1641,6 +1645,10 @@ int gpudb_batch_collect(gpudb_batch* b, uint64_t* rows, void* host, uint64_t hos
             gpudb::setThreadError("batch: collect buffer too small");
             return GPUDB_E_INVALID;
         }
+        B_CHECK(cudaMemsetAsync(counter, 0, 8 * ((size_t)n + 1), b->stream), GPUDB_E_CUDA);
+        kCollect<<<gridFor(b, (const void*)kCollect, 256), 256, 0, b->stream>>>(b->dDesc, b->wlCollect, counter,
+                                                                               counter + 1, dOffs, out);
+        B_CHECK(cudaGetLastError(), GPUDB_E_LAUNCH);
         if (total) B_CHECK(cudaMemcpyAsync(host, out, 24 * total, cudaMemcpyDeviceToHost, b->stream), GPUDB_E_CUDA);
     }
     B_CHECK(cudaEventRecord(b->ev1, b->stream), GPUDB_E_CUDA);

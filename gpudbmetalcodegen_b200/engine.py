@@ -65,10 +65,38 @@ class Result:
         return [dict(zip(self.columns, r)) for r in self.rows]
 
 
+_TEXT_ROWS = 512      # results of up to this many rows come as text, in one call
+_TEXT_BYTES = 1 << 16
+_PARSE = {"i": int, "d": float, "s": str}
+_TYPE = {"i": "int", "d": "double", "s": "string"}
+
+
+def _result_from_text(text: bytes) -> Optional[Result]:
+    """The three texts of gpudb_result_text; None when a cell is quoted."""
+    types, exact, canonical = (t.decode() for t in text.split(b"\0")[:3])
+    if '"' in exact:
+        return None
+    lines = exact.split("\n")
+    columns = lines[0].split(",") if types else []
+    parse = [_PARSE[t] for t in types]
+    rows = [tuple(p(c) for p, c in zip(parse, ln.split(","))) for ln in lines[1:-1]]
+    return Result(columns, [_TYPE[t] for t in types], rows, canonical, exact)
+
+
 def _result_from_c(res) -> Result:
     lib = _lib.load()
     nc, nr = C.c_int(), C.c_longlong()
     lib.gpudb_result_shape(res, C.byref(nc), C.byref(nr))
+    if nr.value <= _TEXT_ROWS and nc.value:
+        buf = C.create_string_buffer(4096)
+        n = lib.gpudb_result_text(res, buf, 4096)
+        if 4096 < n <= _TEXT_BYTES:
+            buf = C.create_string_buffer(n)
+            n = lib.gpudb_result_text(res, buf, n)
+        if 0 < n <= _TEXT_BYTES:
+            r = _result_from_text(C.string_at(buf, n))
+            if r is not None:
+                return r
     names, types = [], []
     for c in range(nc.value):
         buf = C.create_string_buffer(256)
@@ -81,7 +109,7 @@ def _result_from_c(res) -> Result:
         if t == "int":
             out = np.zeros(nr.value, dtype=np.int64)
             if lib.gpudb_result_export_i64(res, c, out.ctypes.data, nr.value) == 0:
-                cols.append([int(v) for v in out])
+                cols.append(out.tolist())
                 continue
             vals = []
             lo, hi = C.c_int64(), C.c_int64()
@@ -160,7 +188,9 @@ class Query:
         self._lib = _lib.load()
         self.spec = spec
         self.tune = tune
-        self.ctx = ctx
+        # the context keeps its prepared queries: a reference back would make
+        # a cycle that only the cyclic collector frees (device memory with it)
+        self._ctx = weakref.ref(ctx) if ctx is not None else None
         if handle is not None:  # prepared elsewhere (an analyzed query)
             self.handle = handle
             return
@@ -168,6 +198,10 @@ class Query:
         st = self._lib.gpudb_query_prepare(ctx.handle if ctx else None, spec.encode(), tune.encode(), C.byref(h))
         check(st, ctx.handle if ctx else None)
         self.handle = h
+
+    @property
+    def ctx(self) -> Optional["Context"]:
+        return self._ctx() if self._ctx is not None else None
 
     @property
     def source(self) -> str:
@@ -210,6 +244,9 @@ class Context:
     def close(self) -> None:
         for q in self._queries.values():
             q.close()
+        self._release()
+
+    def _release(self) -> None:
         self._queries.clear()
         if self.handle:
             self._lib.gpudb_destroy(self.handle)
@@ -223,7 +260,7 @@ class Context:
 
     def __del__(self):
         try:
-            self.close()
+            self._release()  # a query someone still holds stays readable
         except Exception:
             pass
 

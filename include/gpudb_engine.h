@@ -116,6 +116,10 @@ int gpudb_result_export_i64(gpudb_result* r, int col, int64_t* out, long long n)
 const int64_t* gpudb_result_column_data(gpudb_result* r, int col);
 /* GenericResult::toCanonical (%.4f doubles) / full-precision variant. */
 size_t gpudb_result_canonical(gpudb_result* r, int exact, char* buf, size_t cap);
+/* A whole (small) result in one call: three NUL-terminated texts, the column
+ * types (one of i, d, s each), the full-precision form, the canonical form.
+ * Returns the bytes they take; they are written if `cap` holds them. */
+size_t gpudb_result_text(gpudb_result* r, char* buf, size_t cap);
 void gpudb_result_free(gpudb_result* r);
 
 /* Golden comparison (reference: compareCanonical, codegen_main.cpp:63-188).
