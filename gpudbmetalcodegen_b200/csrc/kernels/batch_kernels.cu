@@ -42,7 +42,9 @@ void setThreadError(const std::string& message);
 namespace {
 
 constexpr int kTopK = 16;             // largest k a top-k query may ask for
-constexpr long long kScanChunk = 16384;  // table slots per work item of the passes after the group-by
+// Table slots per work item of the passes after the group-by: 32 items of a
+// table, as far as an item keeps 1024 to 16384 slots.
+constexpr long long kScanMin = 1024, kScanMax = 16384;
 constexpr int kUnroll = 4;            // independent rows in flight per thread
 constexpr int kSmemProbe = 4;         // probes into the shared table before spilling to global
 
@@ -76,6 +78,7 @@ struct QDesc {
     unsigned* bitmap;
     Slot* ht;
     int log2cap, maxProbe;
+    long long scanChunk;
     int aggMode;  // GPUDB_AGG_SHARED / _GLOBAL_WARP / _GLOBAL / _SHARED_DIRECT
     int dense;    // slot i belongs to encoded key i + 1
     unsigned directBase;  // SHARED_DIRECT: the encoded key of shared slot 0
@@ -398,10 +401,10 @@ __global__ void __launch_bounds__(U == 4 ? 1024 : 512, U == 4 ? 1 : 4) kAgg(cons
 //
 // Measured (B200, group stage alone, before -> now; floor: 16 B per row at
 // 6.65 TB/s): 27.1M rows, 71 % pass, 2,838 uniform keys 650 -> 116 us (65);
-// 58.9M rows, 8,763 uniform keys 724 -> 220 (142); 47.9M rows, 57 % pass,
-// Zipf(1.3) keys into 0.6M groups 992 -> 512 (115); 22.8M rows, Zipf over
-// 10,908 keys 302 -> 111 (55); the mixed batch's 34 grouped queries 5.79 ->
-// 3.06 ms. Queries of few keys run at 1.6 x their floor (their loads in
+// 58.9M rows, 8,763 uniform keys 724 -> 221 (142); 47.9M rows, 57 % pass,
+// Zipf(1.3) keys into 0.6M groups 992 -> 348 (115); 22.8M rows, Zipf over
+// 10,908 keys 302 -> 109 (55); the mixed batch's 34 grouped queries 5.79 ->
+// 2.80 ms. Queries of few keys run at 1.6 x their floor (their loads in
 // flight), uniform ones of many keys at the L2's rate of reductions (two per
 // row, 75 G rows/s).
 constexpr int kTableWords = 40;  // of the shared table, per thread
@@ -546,7 +549,11 @@ __device__ __forceinline__ void groupTile(const QDesc& q, const SharedTable& st,
                     cold = false;
                 }
             } else if (PATH == GroupPath::Shared) {
+                // the search ends before the adds: lanes that find their
+                // slot at different probes then add together
+                const unsigned lm = __ballot_sync(0xffffffffu, live);
                 if (live) {
+                    int at = -1;
                     int h = (int)__umulhi(enc * 0x9E3779B1u, (unsigned)st.slots);
 #pragma unroll 1
                     for (int p = 0; p < kSmemProbe; ++p) {
@@ -556,12 +563,14 @@ __device__ __forceinline__ void groupTile(const QDesc& q, const SharedTable& st,
                             cur = prev == 0u ? enc : prev;
                         }
                         if (cur == enc) {
-                            st.add(h, val);
-                            cold = false;
+                            at = h;
                             break;
                         }
                         h = h + 1 < st.slots ? h + 1 : 0;
                     }
+                    __syncwarp(lm);
+                    if (at >= 0) st.add(at, val);
+                    cold = at < 0;
                 }
             } else if (warp) {
                 if (live) {
@@ -597,7 +606,7 @@ template <int U>
 __global__ void __launch_bounds__(1024, 1) kGroup(const QDesc* __restrict__ qs, WorkList wl, long long tile,
                                                   unsigned long long* counter) {
     extern __shared__ unsigned long long groupShared[];
-    __shared__ long long s_item;
+    __shared__ long long s_item[2];
     const int words = kTableWords * (int)blockDim.x;
     SharedTable st{reinterpret_cast<unsigned*>(groupShared), 0};
     unsigned long long* coldV = groupShared + words / 2;
@@ -630,13 +639,21 @@ __global__ void __launch_bounds__(1024, 1) kGroup(const QDesc* __restrict__ qs, 
             if (!direct) *st.key(i) = 0u;
         }
     };
-    for (long long w; (w = pullWork(counter, total, &s_item)) >= 0;) {
+    // Work items are pulled one ahead: the counter's answer arrives while the
+    // current item is processed, and an item costs one barrier.
+    if (threadIdx.x == 0) s_item[0] = (long long)atomicAdd(counter, 1ull);
+    __syncthreads();
+    for (int it = 0;; it ^= 1) {
+        const long long w = s_item[it];
+        if (w >= total) break;
+        long long ahead = 0;
+        if (threadIdx.x == 0) ahead = (long long)atomicAdd(counter, 1ull);
         const int qi = findQuery(wl, w);
         const int qd = __ldg(wl.q + qi);
         if (heldQ >= 0 && heldQ != qd) {
-            // pullWork's barriers ordered every add of the held query before
-            // this flush; the barrier after it orders the reset before the
-            // next rows' adds
+            // the item's closing barrier ordered every add of the held query
+            // before this flush; the barrier after it orders the reset before
+            // the next rows' adds
             flushShared(qs[heldQ]);
             heldQ = -1;
             __syncthreads();
@@ -657,8 +674,10 @@ __global__ void __launch_bounds__(1024, 1) kGroup(const QDesc* __restrict__ qs, 
         } else {
             groupTile<U, GroupPath::Global, false>(q, st, 0u, cq, r0, r1);
         }
+        if (threadIdx.x == 0) s_item[it ^ 1] = ahead;
+        __syncthreads();
     }
-    // pullWork's barriers ordered the last adds before this flush
+    // the closing barriers ordered the last adds before this flush
     if (heldQ >= 0) flushShared(qs[heldQ]);
 }
 
@@ -693,7 +712,7 @@ __global__ void __launch_bounds__(256) kScanGroups(const QDesc* __restrict__ qs,
         const int qi = findQuery(wl, w);
         const QDesc& q = qs[__ldg(wl.q + qi)];
         const long long c = w - __ldg(wl.prefix + qi);
-        const long long i0 = c * kScanChunk, i1 = min(1ll << q.log2cap, i0 + kScanChunk);
+        const long long i0 = c * q.scanChunk, i1 = min(1ll << q.log2cap, i0 + q.scanChunk);
         const bool top = q.tmpl == GPUDB_TPL_TOPK;
         const Slot* __restrict__ ht = q.ht;
         if (threadIdx.x == 0) s_n = 0u;
@@ -797,15 +816,33 @@ __global__ void __launch_bounds__(1024) kStats(const QDesc* __restrict__ qs, Wor
 // Evenly spaced rows of the slice: rows sampled, rows passing the filter,
 // distinct group keys among them and the multiplicity of the most frequent
 // key (the skew signal that picks the aggregation strategy).
+// Latency: a thread's four sample rows load together (filter words, then the
+// keys of those that pass), and the counts are 32-bit (a 64-bit shared add
+// is a compare-and-swap loop, 4,096 of them on one word). B200, four queries
+// of 1M-5M rows: 30 us with 256 threads and 64-bit counts -> 18 us.
 constexpr int kSample = 4096, kSampleSlots = 8192;
 constexpr int kSampleSmem = kSampleSlots * (8 + 4);
-__global__ void kSampleStats(const QDesc* __restrict__ qs, unsigned long long* out /* [n][4] */) {
+constexpr int kSampleThreads = 1024, kSampleRows = kSample / kSampleThreads;
+__global__ void __launch_bounds__(kSampleThreads) kSampleStats(const QDesc* qs, unsigned long long* out /* [n][4] */) {
     extern __shared__ unsigned long long setKeys[];
     unsigned* setCnt = reinterpret_cast<unsigned*>(setKeys + kSampleSlots);
-    __shared__ unsigned long long s_pass, s_distinct;
-    __shared__ unsigned s_top;
+    __shared__ unsigned s_pass, s_distinct, s_top;
     const QDesc& q = qs[blockIdx.x];
-    for (int i = threadIdx.x; i < kSampleSlots; i += blockDim.x) {
+    const long long m = q.rows < kSample ? q.rows : kSample;
+    const bool grouped = q.tmpl == GPUDB_TPL_GROUPBY || q.tmpl == GPUDB_TPL_TOPK;
+    long long r[kSampleRows];
+    bool pass[kSampleRows];
+    int key[kSampleRows];
+#pragma unroll
+    for (int u = 0; u < kSampleRows; ++u) {
+        const long long j = threadIdx.x + u * kSampleThreads;
+        r[u] = j < m ? (j * q.rows) / m : -1;  // evenly spaced rows of the slice
+    }
+#pragma unroll
+    for (int u = 0; u < kSampleRows; ++u) pass[u] = r[u] >= 0 && q.filter[r[u]] < q.thr;
+#pragma unroll
+    for (int u = 0; u < kSampleRows; ++u) key[u] = grouped && pass[u] ? q.key[r[u]] : 0;
+    for (int i = threadIdx.x; i < kSampleSlots; i += kSampleThreads) {
         setKeys[i] = GPUDB_EMPTY64;
         setCnt[i] = 0u;
     }
@@ -815,21 +852,20 @@ __global__ void kSampleStats(const QDesc* __restrict__ qs, unsigned long long* o
         s_top = 0;
     }
     __syncthreads();
-    const long long m = q.rows < kSample ? q.rows : kSample;
-    const bool grouped = q.tmpl == GPUDB_TPL_GROUPBY || q.tmpl == GPUDB_TPL_TOPK;
-    for (long long j = threadIdx.x; j < m; j += blockDim.x) {
-        const long long r = (j * q.rows) / m;  // evenly spaced rows of the slice
-        if (q.filter[r] >= q.thr) continue;
-        atomicAdd(&s_pass, 1ull);
+    unsigned n = 0, fresh = 0;
+#pragma unroll
+    for (int u = 0; u < kSampleRows; ++u) {
+        if (!pass[u]) continue;
+        ++n;
         if (!grouped) continue;
-        const unsigned long long k = (unsigned long long)keyMod(q.key[r], q);
+        const unsigned long long k = (unsigned long long)keyMod(key[u], q);
         unsigned h = (unsigned)gpudb_hash_slot(k, 13);
         for (int p = 0; p < kSampleSlots; ++p) {
             const unsigned long long cur = setKeys[h];
             bool mine = cur == k;
             if (cur == GPUDB_EMPTY64) {
                 const unsigned long long prev = atomicCAS(setKeys + h, GPUDB_EMPTY64, k);
-                if (prev == GPUDB_EMPTY64) atomicAdd(&s_distinct, 1ull);
+                if (prev == GPUDB_EMPTY64) ++fresh;
                 mine = prev == GPUDB_EMPTY64 || prev == k;
             }
             if (mine) {
@@ -839,10 +875,16 @@ __global__ void kSampleStats(const QDesc* __restrict__ qs, unsigned long long* o
             h = (h + 1) & (kSampleSlots - 1);
         }
     }
+    n = __reduce_add_sync(0xffffffffu, n);
+    fresh = __reduce_add_sync(0xffffffffu, fresh);
+    if ((threadIdx.x & 31) == 0) {
+        if (n) atomicAdd(&s_pass, n);
+        if (fresh) atomicAdd(&s_distinct, fresh);
+    }
     __syncthreads();
     unsigned top = 0;
-    for (int i = threadIdx.x; i < kSampleSlots; i += blockDim.x) top = max(top, setCnt[i]);
-    for (int o = 16; o > 0; o >>= 1) top = max(top, __shfl_xor_sync(0xffffffffu, top, o));
+    for (int i = threadIdx.x; i < kSampleSlots; i += kSampleThreads) top = max(top, setCnt[i]);
+    top = __reduce_max_sync(0xffffffffu, top);
     if ((threadIdx.x & 31) == 0) atomicMax(&s_top, top);
     __syncthreads();
     if (threadIdx.x == 0) {
@@ -915,8 +957,8 @@ __global__ void __launch_bounds__(256) kCollect(const QDesc* __restrict__ qs, Wo
             }
         } else {
             // a warp takes 128 slots at a time and reserves its rows with one atomic
-            const long long i1 = min(1ll << q.log2cap, (c + 1) * kScanChunk);
-            for (long long b = c * kScanChunk + (threadIdx.x >> 5) * 128; b < i1; b += 4 * blockDim.x) {
+            const long long i1 = min(1ll << q.log2cap, (c + 1) * q.scanChunk);
+            for (long long b = c * q.scanChunk + (threadIdx.x >> 5) * 128; b < i1; b += 4 * blockDim.x) {
                 Slot s[4];
                 unsigned m[4], n = 0u;
 #pragma unroll
@@ -998,7 +1040,8 @@ struct gpudb_batch {
     // threads per CTA and rows in flight per thread of the group-by kernel.
     // Measured on the 64-query mixed batch (group stage, ms): 512 threads
     // with 1 / 2 / 4 rows 3.92 / 3.62 / 5.08, 1,024 threads 3.39 / 3.06 /
-    // 4.25: the larger CTA holds the larger shared table, four rows spill.
+    // 4.25 (2.80 for 2 rows since the shared search ends before its adds):
+    // the larger CTA holds the larger shared table, four rows spill.
     int groupBlock = 1024, groupRows = 2;
     // rows in flight per thread of the agg / join kernel: 2 (32 registers,
     // every thread slot resident; measured 9.9 ms against 10.6 ms per
@@ -1045,6 +1088,10 @@ void dropGraph(gpudb_batch* b) {
     b->graph = nullptr;
 }
 
+long long scanChunk(unsigned long long cap) {
+    return std::min(kScanMax, std::max<long long>(kScanMin, (long long)cap / 32));
+}
+
 // Lay out the arena and the work lists for the current queries.
 int plan(gpudb_batch* b) {
     const int n = (int)b->queries.size();
@@ -1066,7 +1113,7 @@ int plan(gpudb_batch* b) {
             z += sizeof(Slot) * caps[i];
             if (q.tmpl == GPUDB_TPL_TOPK) {
                 sOff[i] = sc;
-                tkChunks[i] = (long long)((caps[i] + kScanChunk - 1) / kScanChunk);
+                tkChunks[i] = (long long)((caps[i] + scanChunk(caps[i]) - 1) / scanChunk(caps[i]));
                 sc += al256(16 * kTopK * (size_t)tkChunks[i] + 16 * kTopK);
             }
         }
@@ -1082,22 +1129,23 @@ int plan(gpudb_batch* b) {
     b->desc.assign(n, QDesc{});
     std::vector<int> lBuild, lAgg, lGroup, lTopk, lAll(n), lCollect;
     std::vector<long long> pBuild{0}, pAgg{0}, pGroup{0}, pScan{0}, pAll{0}, pCollect{0};
-    // Two work items for each of the 4 x numSMs CTAs of 512 threads before
-    // an item gets the tuning's rows: 8M rows in 32K-row items are work for
-    // 233 of 592 CTAs (B200, four queries of 1M-5M rows: see kGroup)
+    // Two work items for each resident CTA (three of the group-by's larger
+    // ones) before an item gets the tuning's rows: 8M rows in 32K-row items
+    // are work for 233 of 592 CTAs (B200, four queries of 1M-5M rows, group
+    // stage: 192 us in such items by the kernel of that time, 43 us now).
     long long rBuild = 0, rAgg = 0, rGroup = 0;
     for (const auto& q : b->queries) {
         if (q.tmpl == GPUDB_TPL_JOIN) rBuild += (long long)q.dim_rows;
         (grouped(q.tmpl) ? rGroup : rAgg) += (long long)q.rows;
     }
-    auto tileFor = [&](long long rows) {
-        const long long t = (rows / (8ll * b->numSMs) + 1023) / 1024 * 1024;
+    auto tileFor = [&](long long rows, long long items) {
+        const long long t = (rows / items + 1023) / 1024 * 1024;
         return std::min(b->tile, std::max<long long>(4096, t));
     };
-    b->tileBuild = tileFor(rBuild);
-    b->tileAgg = tileFor(rAgg);
-    b->tileGroup = tileFor(rGroup);
-    b->tileStats = tileFor(rAgg + rGroup);
+    b->tileBuild = tileFor(rBuild, 8ll * b->numSMs);
+    b->tileAgg = tileFor(rAgg, 8ll * b->numSMs);
+    b->tileGroup = tileFor(rGroup, 3ll * b->numSMs * std::max(1, 1024 / b->groupBlock));
+    b->tileStats = tileFor(rAgg + rGroup, 8ll * b->numSMs);
     for (int i = 0; i < n; i++) {
         const auto& q = b->queries[i];
         QDesc& d = b->desc[i];
@@ -1147,6 +1195,7 @@ int plan(gpudb_batch* b) {
             p = zb + al256((size_t)(p - zb));
             d.ht = reinterpret_cast<Slot*>(p);
             d.log2cap = log2u(caps[i]);
+            d.scanChunk = scanChunk(caps[i]);
             // no probe and no overflow where the table can hold every key anyway
             d.dense = 2 * (unsigned long long)d.card - 1 <= caps[i];
             if (q.tmpl == GPUDB_TPL_TOPK) {
@@ -1166,7 +1215,7 @@ int plan(gpudb_batch* b) {
             lAgg.push_back(i);
             pAgg.push_back(pAgg.back() + items(d.rows, b->tileAgg));
         }
-        const long long chunks = items((long long)caps[i], kScanChunk);
+        const long long chunks = caps[i] ? items((long long)caps[i], d.scanChunk) : 0;
         if (grouped(q.tmpl)) {
             lGroup.push_back(i);
             pGroup.push_back(pGroup.back() + items(d.rows, b->tileGroup));
@@ -1558,7 +1607,7 @@ int gpudb_batch_features(gpudb_batch* b, float* f, double* ms) {
     if (int st = b->sample.reserve(32 * (size_t)n, b->stream)) return st;
     unsigned long long* out = static_cast<unsigned long long*>(b->sample.p);
     B_CHECK(cudaEventRecord(b->ev0, b->stream), GPUDB_E_CUDA);
-    kSampleStats<<<n, 256, kSampleSmem, b->stream>>>(b->dDesc, out);
+    kSampleStats<<<n, kSampleThreads, kSampleSmem, b->stream>>>(b->dDesc, out);
     B_CHECK(cudaGetLastError(), GPUDB_E_LAUNCH);
     B_CHECK(cudaEventRecord(b->ev1, b->stream), GPUDB_E_CUDA);
     std::vector<unsigned long long> h(4 * (size_t)n);
