@@ -214,6 +214,63 @@ __device__ __forceinline__ unsigned long long gpudb_warp_reserve(unsigned long l
 }
 
 // ------------------------------------------------------------------
+// List entries past a block's own buffer: each warp reserves `chunk` (>= 32)
+// of them at a time and hands them out from its own word in shared memory
+// (initially `chunk`), which packs the chunk's first position and the entries
+// handed out. The lanes that arrive together take theirs with one add; the
+// group that uses the chunk up reserves the next one, and a group that
+// arrives meanwhile reserves just its own entries. At the end the block moves
+// entries of its buffer into what is left of its warps' chunks, so the list
+// has no holes: 32 chunks fit the buffer, which is full by then.
+// One atomic on the counter per entry is 5.5 G/s on B200 (one address), so a
+// kernel with 6M entries took 1.08 ms for them alone.
+// ------------------------------------------------------------------
+#define GPUDB_LIST_SHIFT 16
+#define GPUDB_LIST_USED 0xffffull
+
+__device__ __forceinline__ unsigned long long gpudb_list_pos(unsigned long long* words, unsigned chunk,
+                                                             unsigned long long* counter) {
+    const unsigned m = __activemask();
+    const unsigned lane = threadIdx.x & 31u;
+    const int leader = __ffs(m) - 1;
+    const unsigned n = __popc(m), rank = __popc(m & ((1u << lane) - 1u));
+    unsigned long long w = 0, next = 0;
+    if ((int)lane == leader) {
+        unsigned long long* word = words + (threadIdx.x >> 5);
+        w = atomicAdd(word, (unsigned long long)n);
+        const unsigned used = (unsigned)(w & GPUDB_LIST_USED);
+        if (used > chunk) {
+            next = atomicAdd(counter, (unsigned long long)n);
+        } else if (used + n > chunk) {
+            next = atomicAdd(counter, (unsigned long long)chunk);
+            atomicExch(word, (next << GPUDB_LIST_SHIFT) | (unsigned long long)(used + n - chunk));
+        }
+    }
+    w = __shfl_sync(m, w, leader);
+    next = __shfl_sync(m, next, leader);
+    const unsigned used = (unsigned)(w & GPUDB_LIST_USED);
+    if (used > chunk) return next + rank;
+    if (used + rank < chunk) return (w >> GPUDB_LIST_SHIFT) + used + rank;
+    return next + (used + rank - chunk);
+}
+// After a block barrier: positions left in the block's chunks, and the
+// position of buffer entry `i` (the leftovers first, then from `base`).
+__device__ __forceinline__ unsigned gpudb_list_left(const unsigned long long* words, unsigned chunk) {
+    unsigned left = 0;
+    for (unsigned v = 0; v < (blockDim.x + 31u) / 32u; ++v) left += chunk - (unsigned)(words[v] & GPUDB_LIST_USED);
+    return left;
+}
+__device__ __forceinline__ unsigned long long gpudb_list_place(const unsigned long long* words, unsigned chunk,
+                                                               unsigned i, unsigned long long base) {
+    for (unsigned v = 0; v < (blockDim.x + 31u) / 32u; ++v) {
+        const unsigned used = (unsigned)(words[v] & GPUDB_LIST_USED), left = chunk - used;
+        if (i < left) return (words[v] >> GPUDB_LIST_SHIFT) + used + i;
+        i -= left;
+    }
+    return base + i;
+}
+
+// ------------------------------------------------------------------
 // V consecutive elements of a staged column (shared memory, aligned to
 // sizeof(T) * V) into registers with as few wide loads as possible.
 // ------------------------------------------------------------------

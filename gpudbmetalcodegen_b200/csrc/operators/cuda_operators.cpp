@@ -1240,14 +1240,17 @@ void CudaMaterialize::produce(CudaCodegen& cg, ConsumerFn consume) {
         // 8 KB of shared memory: 2048 rows of one column or 1024 of two
         const int nc = (int)columns_.size();
         const int kBuf = 2048 / nc;
-        const int bo = cg.allocDynamicSmem(kBuf * 4 * nc + 16);
+        const int kChunk = kBuf / 32;  // per warp, of the list positions past the buffer
+        const int bo = cg.allocDynamicSmem(kBuf * 4 * nc + 16 + 32 * 8);
         for (int k = 0; k < nc; k++)
             cg.addLine(columns_[k].type + "* _mb_buf" + S(k) + " = reinterpret_cast<" + columns_[k].type +
                        "*>(gpudb_smem + " + S(bo + k * kBuf * 4) + ");");
         cg.addLine("unsigned* _mb_n = reinterpret_cast<unsigned*>(gpudb_smem + " + S(bo + nc * kBuf * 4) + ");");
         cg.addLine("unsigned long long* _mb_base = reinterpret_cast<unsigned long long*>(gpudb_smem + " +
                    S(bo + nc * kBuf * 4 + 8) + ");");
+        cg.addLine("unsigned long long* _mb_chunk = _mb_base + 1;");
         cg.addLine("if (threadIdx.x == 0) *_mb_n = 0u;");
+        cg.addLine("for (unsigned _w = threadIdx.x; _w < 32u; _w += blockDim.x) _mb_chunk[_w] = " + S(kChunk) + "ull;");
         cg.addLine("__syncthreads();");
         child_->produce(cg, [&]() {
             cg.addLine("const unsigned _mp = atomicAdd(_mb_n, 1u);");
@@ -1257,7 +1260,8 @@ void CudaMaterialize::produce(CudaCodegen& cg, ConsumerFn consume) {
             }, " else {");
             cg.increaseIndent();
             cg.addComment("the CTA's buffer is full: this row goes straight to the list");
-            cg.addLine("const unsigned long long _pos = atomicAdd(" + counterName_ + ", 1ull);");
+            cg.addLine("const unsigned long long _pos = gpudb_list_pos(_mb_chunk, " + S(kChunk) + "u, " + counterName_ +
+                       ");");
             cg.addBlock("if (_pos < (unsigned long long)cap_" + counterName_ + ")", [&]() {
                 for (const auto& c : columns_)
                     cg.addLine(c.arrayName + "[_pos] = (" + c.type + ")(" + c.valueExpr + ");");
@@ -1274,11 +1278,14 @@ void CudaMaterialize::produce(CudaCodegen& cg, ConsumerFn consume) {
         cg.addLine("__syncthreads();");
         cg.addBlock("", [&]() {
             cg.addLine("const unsigned _mn = min(*_mb_n, " + S(kBuf) + "u);");
-            cg.addLine("if (threadIdx.x == 0) *_mb_base = _mn ? atomicAdd(" + counterName_ +
-                       ", (unsigned long long)_mn) : 0ull;");
+            cg.addLine("const unsigned _mleft = *_mb_n > " + S(kBuf) + "u ? gpudb_list_left(_mb_chunk, " + S(kChunk) +
+                       "u) : 0u;");
+            cg.addLine("if (threadIdx.x == 0) *_mb_base = _mn > _mleft ? atomicAdd(" + counterName_ +
+                       ", (unsigned long long)(_mn - _mleft)) : 0ull;");
             cg.addLine("__syncthreads();");
             cg.addBlock("for (unsigned _w = threadIdx.x; _w < _mn; _w += blockDim.x)", [&]() {
-                cg.addLine("const unsigned long long _pos = *_mb_base + _w;");
+                cg.addLine("const unsigned long long _pos = _mleft ? gpudb_list_place(_mb_chunk, " + S(kChunk) +
+                           "u, _w, *_mb_base) : *_mb_base + _w;");
                 cg.addBlock("if (_pos < (unsigned long long)cap_" + counterName_ + ")", [&]() {
                     for (int k = 0; k < nc; k++)
                         cg.addLine(columns_[k].arrayName + "[_pos] = _mb_buf" + S(k) + "[_w];");
@@ -1415,7 +1422,8 @@ static void emitHashMainUpdate(CudaCodegen& cg, const std::string& table, const 
             cg.addBlock("if (_gnew)", [&]() {  // group created
                 cg.addLine("const unsigned _gp = atomicAdd(_gl_n, 1u);");
                 cg.addLine("if (_gp < " + S(kSlotBuf) + "u) _gl_buf[_gp] = (unsigned)_gslot;");
-                cg.addLine("else " + list + "[atomicAdd(" + nlist + ", 1ull)] = (unsigned)_gslot;");
+                cg.addLine("else " + list + "[gpudb_list_pos(_gl_chunk, " + S(kSlotBuf / 32) + "u, " + nlist +
+                           ")] = (unsigned)_gslot;");
             });
         else if (slotList == 2)
             cg.addLine("if (_gnew) " + list + "[atomicAdd(" + nlist + ", 1ull)] = (unsigned)_gslot;");
@@ -1495,12 +1503,15 @@ void CudaHashGroupBy::produce(CudaCodegen& cg, ConsumerFn consume) {
     if (slotList_) {
         cg.addBufferParam(list, "unsigned", cap, false);
         cg.addAtomicBufferParam(nlist, "unsigned long long", "1");
-        const int bo = cg.allocDynamicSmem(kSlotBuf * 4 + 16);
+        const int bo = cg.allocDynamicSmem(kSlotBuf * 4 + 16 + 32 * 8);
         cg.addLine("unsigned* _gl_buf = reinterpret_cast<unsigned*>(gpudb_smem + " + S(bo) + ");");
         cg.addLine("unsigned* _gl_n = _gl_buf + " + S(kSlotBuf) + ";");
         cg.addLine("unsigned long long* _gl_base = reinterpret_cast<unsigned long long*>(_gl_buf + " + S(kSlotBuf + 2) +
                    ");");
+        cg.addLine("unsigned long long* _gl_chunk = _gl_base + 1;");
         cg.addLine("if (threadIdx.x == 0) *_gl_n = 0u;");
+        cg.addLine("for (unsigned _w = threadIdx.x; _w < 32u; _w += blockDim.x) _gl_chunk[_w] = " + S(kSlotBuf / 32) +
+                   "ull;");
         cg.addLine("__syncthreads();");
     }
     std::vector<std::string> aggNames;
@@ -1584,10 +1595,14 @@ void CudaHashGroupBy::produce(CudaCodegen& cg, ConsumerFn consume) {
         cg.addLine("__syncthreads();");
         cg.addBlock("", [&]() {
             cg.addLine("const unsigned _gn = min(*_gl_n, " + S(kSlotBuf) + "u);");
-            cg.addLine("if (threadIdx.x == 0) *_gl_base = _gn ? atomicAdd(" + nlist + ", (unsigned long long)_gn) : 0ull;");
+            cg.addLine("const unsigned _gleft = *_gl_n > " + S(kSlotBuf) + "u ? gpudb_list_left(_gl_chunk, " +
+                       S(kSlotBuf / 32) + "u) : 0u;");
+            cg.addLine("if (threadIdx.x == 0) *_gl_base = _gn > _gleft ? atomicAdd(" + nlist +
+                       ", (unsigned long long)(_gn - _gleft)) : 0ull;");
             cg.addLine("__syncthreads();");
             cg.addLine("for (unsigned _w = threadIdx.x; _w < _gn; _w += blockDim.x) " + list +
-                       "[*_gl_base + _w] = _gl_buf[_w];");
+                       "[_gleft ? gpudb_list_place(_gl_chunk, " + S(kSlotBuf / 32) + "u, _w, *_gl_base) : *_gl_base + _w]"
+                       " = _gl_buf[_w];");
         });
     }
     auto& hs = cg.resultSchema();
