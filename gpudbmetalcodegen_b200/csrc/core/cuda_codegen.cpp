@@ -313,12 +313,13 @@ std::string CudaCodegen::print() {
     std::ostringstream out;
     out << kDeviceHeader << "\n";
     if (!helperCode_.empty()) out << "// --- plan helpers ---\n" << helperCode_ << "\n";
+    if (phases_.size() > kMaxPhases) throw std::runtime_error("CudaCodegen::print: too many phases");
     for (size_t pi = 0; pi < phases_.size(); pi++) {
         assignArgIndices(phases_[pi]);
         const auto& ph = phases_[pi];
         out << "\n// === Phase " << pi << ": " << ph.name << " ===\n";
         out << generateSignature(ph) << " {\n";
-        out << "    GPUDB_THREAD_VARS\n";
+        out << "    GPUDB_THREAD_VARS\n    GPUDB_PHASE_START(" << pi << ")\n";
         if (ph.dynamicSmemBytes > 0) out << "    extern __shared__ __align__(1024) unsigned char gpudb_smem[];\n";
         out << ph.code;
         out << "}\n";

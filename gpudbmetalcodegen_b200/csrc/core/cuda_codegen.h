@@ -32,6 +32,8 @@ using ConsumerFn = std::function<void()>;
 
 class CudaCodegen {
 public:
+    static constexpr size_t kMaxPhases = 1024;  // start times kept beside the error word
+
     // ---- code emission -------------------------------------------------
     void addLine(const std::string& line);
     void addBlock(const std::string& header, const std::function<void()>& body,

@@ -43,11 +43,12 @@ CudaGenericExecutor::CudaGenericExecutor(int device) : device_(device) {
     GPUDB_CUDA_OR_THROW(cudaSetDevice(device));
     GPUDB_CUDA_OR_THROW(cudaDeviceGetAttribute(&numSMs_, cudaDevAttrMultiProcessorCount, device));
     GPUDB_CUDA_OR_THROW(cudaStreamCreateWithFlags(&stream_, cudaStreamNonBlocking));
-    GPUDB_CUDA_OR_THROW(cudaMalloc((void**)&errWord_, sizeof(unsigned)));
-    GPUDB_CUDA_OR_THROW(cudaMemset(errWord_, 0, sizeof(unsigned)));
+    GPUDB_CUDA_OR_THROW(cudaMalloc((void**)&errWord_, kErrBytes));
+    GPUDB_CUDA_OR_THROW(cudaMemset(errWord_, 0, kErrBytes));
     // the error word's copy and the staging area share one pinned block
-    GPUDB_CUDA_OR_THROW(cudaHostAlloc((void**)&stageHost_, kStageBytes + 64, cudaHostAllocDefault));
+    GPUDB_CUDA_OR_THROW(cudaHostAlloc((void**)&stageHost_, kStageBytes + kErrBytes, cudaHostAllocDefault));
     errHost_ = reinterpret_cast<unsigned*>(stageHost_ + kStageBytes);
+    for (auto& e : events_) GPUDB_CUDA_OR_THROW(cudaEventCreate(&e));
     const DriverApi& api = driverApi();
     if (!api.loaded) throw std::runtime_error("CUDA driver API unavailable: " + api.error);
 }
@@ -60,7 +61,8 @@ CudaGenericExecutor::~CudaGenericExecutor() {
     for (auto& [_, b] : ownedColumns_)
         if (b.ptr) cudaFree(b.ptr);
     ownedColumns_.clear();
-    for (auto e : events_) cudaEventDestroy(e);
+    for (auto e : events_)
+        if (e) cudaEventDestroy(e);
     if (errWord_) cudaFree(errWord_);
     if (stageHost_) cudaFreeHost(stageHost_);
     if (stream_) cudaStreamDestroy(stream_);
@@ -328,14 +330,6 @@ GenericResult CudaGenericExecutor::collectResult(const CudaResultSchema& schema)
 // ---------------------------------------------------------------------------
 // launch preparation
 // ---------------------------------------------------------------------------
-void CudaGenericExecutor::ensureEvents(size_t n) {
-    while (events_.size() < n) {
-        cudaEvent_t e;
-        GPUDB_CUDA_OR_THROW(cudaEventCreate(&e));
-        events_.push_back(e);
-    }
-}
-
 bool CudaGenericExecutor::buildLaunch(const RuntimeCompiler::CompiledQuery& cq, const CudaCodegen::PhaseInfo& ph,
                                       Launch& l, std::string& error) {
     const DriverApi& api = driverApi();
@@ -518,7 +512,6 @@ int CudaGenericExecutor::execute(const RuntimeCompiler::CompiledQuery& cq,
     }
 
     const size_t nl = launches.size();
-    ensureEvents(nl + 1);
     staged_.clear();
     out.phaseNames.clear();
     out.phaseTimesMs.assign(nl, 0.0);
@@ -534,8 +527,8 @@ int CudaGenericExecutor::execute(const RuntimeCompiler::CompiledQuery& cq,
     out.launches = (long long)nl;
     out.totalKernelTimeMs = 0.0;
 
-    // Timed iterations record an event after the fills and one after every
-    // kernel: a phase's time runs from the event before it to its own.
+    // Timed iterations record an event after the fills and one after the
+    // last kernel.
     auto launchAll = [&](bool timed) -> bool {
         if (fillBuffers(fills, stream_) != cudaSuccess) {
             error = "buffer fill failed";
@@ -555,8 +548,8 @@ int CudaGenericExecutor::execute(const RuntimeCompiler::CompiledQuery& cq,
                 error = "launch of '" + l.name + "' failed: " + cuErrorString(r);
                 return false;
             }
-            if (timed) cudaEventRecord(events_[i + 1], stream_);
         }
+        if (timed) cudaEventRecord(events_[1], stream_);
         return true;
     };
 
@@ -624,17 +617,12 @@ int CudaGenericExecutor::execute(const RuntimeCompiler::CompiledQuery& cq,
     const bool stage = !defer && last == (int)phases.size();
     unsigned bits = 0;
     auto wait = [&](int iter, const char* what) -> bool {
-        cudaError_t e;
-        if (iter == total - 1) {
-            if (!stage) stageSchema_ = nullptr;
-            if (!enqueueTail()) {
-                error = "cannot read the device error word";
-                return false;
-            }
-            e = cudaStreamSynchronize(stream_);
-        } else {
-            e = cudaEventSynchronize(events_[nl]);
+        if (iter == total - 1 && !stage) stageSchema_ = nullptr;
+        if (!enqueueTail(iter == total - 1, phases.size())) {
+            error = "cannot read the device error word";
+            return false;
         }
+        const cudaError_t e = cudaStreamSynchronize(stream_);
         if (e != cudaSuccess) error = cudaErr(what, e);
         return e == cudaSuccess;
     };
@@ -647,20 +635,26 @@ int CudaGenericExecutor::execute(const RuntimeCompiler::CompiledQuery& cq,
                 error = "cudaGraphLaunch failed";
                 return -6;
             }
-            if (timed) cudaEventRecord(events_[nl], stream_);
+            if (timed) cudaEventRecord(events_[1], stream_);
         } else if (!launchAll(timed)) {
             return -6;
         }
         if (!timed) continue;
         if (!wait(iter, it != graphs_.end() ? "graph replay" : "kernel execution")) return -7;
         float ms = 0;
-        if (it == graphs_.end())
-            for (size_t i = 0; i < nl; i++) {
-                cudaEventElapsedTime(&ms, events_[i], events_[i + 1]);
-                out.phaseTimesMs[i] += ms / measured;
+        cudaEventElapsedTime(&ms, events_[0], events_[1]);
+        out.totalKernelTimeMs += (double)ms / measured;
+        if (it == graphs_.end()) {
+            // a phase ends where the next one starts, the last with the run
+            const uint64_t* start = reinterpret_cast<const uint64_t*>(errHost_) + 1 + first;
+            double rest = ms;
+            for (size_t i = 0; i + 1 < nl; i++) {
+                const double t = std::min(rest, start[i + 1] > start[i] ? (start[i + 1] - start[i]) * 1e-6 : 0.0);
+                out.phaseTimesMs[i] += t / measured;
+                rest -= t;
             }
-        cudaEventElapsedTime(&ms, events_[0], events_[nl]);
-        out.totalKernelTimeMs += ms / measured;
+            out.phaseTimesMs[nl - 1] += rest / measured;
+        }
     }
     if (defer) {
         pendingErr_ = true;
@@ -679,20 +673,22 @@ void CudaGenericExecutor::stageResult(const CudaResultSchema* schema) {
 
 // Enqueue the copies that follow a run's last kernel: the error word, and
 // the requested result buffers as far as they fit the staging area.
-bool CudaGenericExecutor::enqueueTail() {
-    if (stageSchema_) {
+// What the host reads after a run, in one launch: the error word with the
+// phases' start times, and the small buffers of a `result`.
+bool CudaGenericExecutor::enqueueTail(bool result, size_t phases) {
+    std::vector<BufferRead> reads{{errWord_, errHost_, 8 + 8 * phases}};
+    if (result && stageSchema_) {
         size_t at = 0;
         for (const auto& [name, bytes] : CudaResultCollector::smallReads(
                  *stageSchema_, [this](const std::string& e) { return resolver_.resolve(e); }, kStageBytes)) {
             auto b = buffers_.find(name);
             if (b == buffers_.end() || !b->second.ptr || bytes > b->second.bytes || at + bytes > kStageBytes) continue;
-            if (cudaMemcpyAsync(stageHost_ + at, b->second.ptr, bytes, cudaMemcpyDeviceToHost, stream_) != cudaSuccess)
-                return false;
+            reads.push_back({b->second.ptr, stageHost_ + at, bytes});
             staged_.push_back({name, bytes, at});
             at += (bytes + 15) & ~size_t(15);
         }
     }
-    return cudaMemcpyAsync(errHost_, errWord_, sizeof(unsigned), cudaMemcpyDeviceToHost, stream_) == cudaSuccess;
+    return readBuffers(reads, stream_) == cudaSuccess;
 }
 
 // The error bits that enqueueTail() brought (the stream has been waited for).

@@ -12,7 +12,9 @@
 //   * one CUDA stream per executor; all fills (one launch) and kernels are
 //     stream-ordered, the host synchronises once per execute(), and the
 //     error word and a small result come back under that same wait;
-//   * per-phase CUDA events (the reference's GPU timestamps);
+//   * a run is timed by two CUDA events, its phases by the start time that
+//     each kernel writes beside the error word (the reference's GPU
+//     timestamps);
 //   * launch = min(work, SMs x occupancy) persistent CTAs, with the
 //     dynamic shared memory each phase declares (TMA ring, smem tables);
 //   * the device error word is cleared before and read after each run;
@@ -152,8 +154,9 @@ private:
     int device_ = 0;
     int numSMs_ = 148;
     cudaStream_t stream_ = nullptr;
-    unsigned* errWord_ = nullptr;
+    unsigned* errWord_ = nullptr;  // the error word; from byte 8 on, the phases' start times (ns)
     unsigned* errHost_ = nullptr;
+    static constexpr size_t kErrBytes = 8 + 8 * CudaCodegen::kMaxPhases;
     static constexpr size_t kMaxGraphs = 512;  // captured graphs kept per context
     bool skipZeroInit_ = false;
     bool useGraphs_ = false;
@@ -171,7 +174,7 @@ private:
     std::map<std::pair<uint64_t, CUfunction>, int> carveoutSet_;
     // blocks per SM of (load id, function, block, dynamic shared memory)
     std::map<std::tuple<uint64_t, CUfunction, unsigned, unsigned>, int> occupancy_;
-    std::vector<cudaEvent_t> events_;
+    cudaEvent_t events_[2] = {nullptr, nullptr};  // around a timed iteration's kernels
     // pinned copies of the buffers a result is decoded from
     struct Staged {
         std::string name;
@@ -181,7 +184,7 @@ private:
     char* stageHost_ = nullptr;
     const CudaResultSchema* stageSchema_ = nullptr;
     std::vector<Staged> staged_;
-    bool enqueueTail();
+    bool enqueueTail(bool result, size_t phases);
     bool finishTail(unsigned& bits, std::string& error);
     GroupWorkspace groupScratch_;  // device scratch of group collection, grown on demand
     struct GraphEntry {
@@ -193,7 +196,6 @@ private:
     std::unordered_set<std::string> seenOnce_;    // keys run once, eagerly, not captured yet
     static constexpr size_t kMaxSeen = 4096;
 
-    void ensureEvents(size_t n);
     bool allocateBuffers(const CudaCodegen::PhaseInfo& phase, std::string& error);
     bool buildLaunch(const RuntimeCompiler::CompiledQuery& cq, const CudaCodegen::PhaseInfo& phase, Launch& l,
                      std::string& error);

@@ -1,5 +1,6 @@
 #pragma once
-// One launch for all of a run's buffer fills (kernels/fill.cu).
+// One launch for all of a run's buffer fills, one for what it reads back
+// (kernels/fill.cu).
 #include <cuda_runtime.h>
 
 #include <cstddef>
@@ -17,5 +18,16 @@ struct BufferFill {
 // buffers each, instead of a memset per buffer.
 constexpr int kFillSegments = 32;
 cudaError_t fillBuffers(const std::vector<BufferFill>& fills, cudaStream_t stream);
+
+struct BufferRead {
+    const void* src;  // device memory
+    void* dst;        // pinned host memory
+    size_t bytes;
+};
+
+// Enqueue small reads: the kernel writes the host memory itself, up to
+// kReadSegments buffers a launch, instead of a copy per buffer.
+constexpr int kReadSegments = 32;
+cudaError_t readBuffers(const std::vector<BufferRead>& reads, cudaStream_t stream);
 
 }  // namespace gpudb

@@ -1,4 +1,5 @@
-// A run's buffer fills in one launch (execution/fill.h). A plan fills up to
+// A run's buffer fills in one launch, its small reads in another
+// (execution/fill.h). A plan fills up to
 // a dozen small buffers (counters, ticket words, bitmaps, output lists), and
 // a memset costs about 2 us of stream time each, whatever its size: the
 // join's nine took 17 us of a 600K-row query whose kernels take 50 (B200);
@@ -37,7 +38,43 @@ __global__ void __launch_bounds__(kThreads) kFill(const __grid_constant__ Segmen
     }
 }
 
+struct Reads {
+    const unsigned char* src[kReadSegments];
+    unsigned char* dst[kReadSegments];
+    unsigned long long bytes[kReadSegments];
+};
+
+// One block per buffer. A copy of a few bytes is about 3 us of stream time
+// and 2 us of the host's; a run reads back its error word, its phases' start
+// times and one to five result buffers.
+__global__ void __launch_bounds__(kThreads) kRead(const __grid_constant__ Reads r) {
+    const unsigned char* src = r.src[blockIdx.x];
+    unsigned char* dst = r.dst[blockIdx.x];
+    const unsigned long long n = r.bytes[blockIdx.x];
+    const unsigned long long body =
+        (reinterpret_cast<size_t>(src) | reinterpret_cast<size_t>(dst)) % 8 ? 0ull : n / 8 * 8;
+    for (unsigned long long i = 8ull * threadIdx.x; i < body; i += 8ull * kThreads)
+        *reinterpret_cast<unsigned long long*>(dst + i) = *reinterpret_cast<const unsigned long long*>(src + i);
+    for (unsigned long long i = body + threadIdx.x; i < n; i += kThreads) dst[i] = src[i];
+}
+
 }  // namespace
+
+cudaError_t readBuffers(const std::vector<BufferRead>& reads, cudaStream_t stream) {
+    for (size_t at = 0; at < reads.size(); at += kReadSegments) {
+        Reads r{};
+        const unsigned n = (unsigned)std::min<size_t>(kReadSegments, reads.size() - at);
+        for (unsigned i = 0; i < n; ++i) {
+            r.src[i] = static_cast<const unsigned char*>(reads[at + i].src);
+            r.dst[i] = static_cast<unsigned char*>(reads[at + i].dst);
+            r.bytes[i] = reads[at + i].bytes;
+        }
+        kRead<<<n, kThreads, 0, stream>>>(r);
+        const cudaError_t e = cudaGetLastError();
+        if (e != cudaSuccess) return e;
+    }
+    return cudaSuccess;
+}
 
 cudaError_t fillBuffers(const std::vector<BufferFill>& fills, cudaStream_t stream) {
     Segments s{};
