@@ -274,7 +274,7 @@ void CudaGenericExecutor::releaseAllocatedBuffers() {
 
 // The groups of a hash aggregate are compacted, ordered and made columns on
 // the device; where device scratch cannot be had the host walks the table.
-bool CudaGenericExecutor::collectGroupsOnDevice(const CudaResultSchema& schema, GenericResult& r) {
+GroupTable CudaGenericExecutor::groupTable(const CudaResultSchema& schema) const {
     const auto& h = schema.hashAgg;
     GroupTable t;
     t.cap = resolver_.resolve(h.capacitySymbol);
@@ -293,11 +293,18 @@ bool CudaGenericExecutor::collectGroupsOnDevice(const CudaResultSchema& schema, 
         t.packedStride = 0;
         for (const auto& a : h.aggs) t.aggs.push_back(buffer(a.buffer, t.cap * 8));
     }
+    return t;
+}
+
+bool CudaGenericExecutor::collectGroupsOnDevice(const CudaResultSchema& schema, GenericResult& r) {
+    const auto& h = schema.hashAgg;
     uint64_t rows = 0;
     const int64_t* data = nullptr;
-    std::shared_ptr<HostBlock> host;
+    std::shared_ptr<HostBlock> host = std::move(stagedGroups_);
     std::string error;
-    if (!collectGroups(t, h.sortByKey, groupScratch_, stream_, rows, data, host, error)) {
+    if (host) {
+        smallGroups(*host, rows, data);
+    } else if (!collectGroups(groupTable(schema), h.sortByKey, groupScratch_, stream_, rows, data, host, error)) {
         if (!error.empty()) throw std::runtime_error("collector: " + error);
         return false;
     }
@@ -513,6 +520,7 @@ int CudaGenericExecutor::execute(const RuntimeCompiler::CompiledQuery& cq,
 
     const size_t nl = launches.size();
     staged_.clear();
+    stagedGroups_.reset();
     out.phaseNames.clear();
     out.phaseTimesMs.assign(nl, 0.0);
     out.phaseGrid.clear();
@@ -669,6 +677,7 @@ int CudaGenericExecutor::execute(const RuntimeCompiler::CompiledQuery& cq,
 void CudaGenericExecutor::stageResult(const CudaResultSchema* schema) {
     stageSchema_ = schema;
     staged_.clear();
+    stagedGroups_.reset();
 }
 
 // Enqueue the copies that follow a run's last kernel: the error word, and
@@ -688,7 +697,19 @@ bool CudaGenericExecutor::enqueueTail(bool result, size_t phases) {
             at += (bytes + 15) & ~size_t(15);
         }
     }
-    return readBuffers(reads, stream_) == cudaSuccess;
+    if (readBuffers(reads, stream_) != cudaSuccess) return false;
+    if (result && stageSchema_ && stageSchema_->kind == CudaResultSchema::HASH_AGG) {
+        // the groups of a small table follow their kernels without a wait
+        // between; a table that cannot be had or is larger is collected later
+        std::string error;
+        try {
+            enqueueSmallGroups(groupTable(*stageSchema_), stageSchema_->hashAgg.sortByKey, groupScratch_, stream_,
+                               stagedGroups_, error);
+        } catch (const std::exception&) {
+        }
+        return error.empty();
+    }
+    return true;
 }
 
 // The error bits that enqueueTail() brought (the stream has been waited for).

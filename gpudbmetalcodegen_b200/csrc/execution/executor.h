@@ -184,6 +184,8 @@ private:
     char* stageHost_ = nullptr;
     const CudaResultSchema* stageSchema_ = nullptr;
     std::vector<Staged> staged_;
+    std::shared_ptr<HostBlock> stagedGroups_;  // a small table's groups, enqueued with the run
+    GroupTable groupTable(const CudaResultSchema& schema) const;
     bool enqueueTail(bool result, size_t phases);
     bool finishTail(unsigned& bits, std::string& error);
     GroupWorkspace groupScratch_;  // device scratch of group collection, grown on demand

@@ -59,4 +59,12 @@ struct GroupWorkspace {
 bool collectGroups(const GroupTable& t, bool sorted, GroupWorkspace& ws, cudaStream_t stream, uint64_t& rows,
                    const int64_t*& data, std::shared_ptr<HostBlock>& host, std::string& error);
 
+// The same for a table of few slots, enqueued on `stream` without a wait:
+// smallGroups() reads the columns once the stream has been waited for. False
+// (with `error` empty) when the table is too large or there is no scratch or
+// no pinned memory for it.
+bool enqueueSmallGroups(const GroupTable& t, bool sorted, GroupWorkspace& ws, cudaStream_t stream,
+                        std::shared_ptr<HostBlock>& host, std::string& error);
+void smallGroups(const HostBlock& host, uint64_t& rows, const int64_t*& data);
+
 }  // namespace gpudb

@@ -5,13 +5,15 @@
 // host pass over its slots, a host sort and a row object per group. Measured
 // on B200, whole calls: a hash join with 2^20 keys 350 ms before, 1.71 ms
 // now (0.8 ms of it the join's kernels, 0.5 ms the 25 MB over the link); a
-// group-by with 4,099 groups 788 us before, 167 us now.
+// group-by with 4,099 groups 788 us before, 80 us now.
 //
-// Tables of at most kSmallCap slots take three launches: compaction, a rank
-// sort (group keys are distinct, so a key's position is the number of
-// smaller keys; n^2 compares over the whole GPU, 16.8M for 4,099 groups) and
-// a pass that writes the columns straight into the mapped host block, so the
-// host waits once.
+// Tables of at most kSmallCap slots follow the query's own kernels without a
+// wait between: compaction, key order (group keys are distinct, so a key's
+// position is the number of smaller keys: few keys are compared with all
+// others, more are sorted by chunks and then searched for in the other
+// chunks) and a pass that writes the columns straight into the mapped host
+// block. With a wait between, and one CTA for all comparisons of a key, the
+// call with 4,099 groups took 119 us.
 // Larger ones count first (the scratch is sized by the groups, not by the
 // slots), then compact, sort the key with its slot number by a
 // least-significant-digit radix sort and gather the aggregates in order.
@@ -31,8 +33,22 @@ namespace gpudb {
 
 namespace {
 
-constexpr uint64_t kSmallCap = 1 << 15;  // 2^15 slots hold at most 2^14 groups at the planned load of 1/2
+// Slots of a small table (at most 2^18 groups at the planned load of 1/2).
+// Whole calls on B200, as a small table / as a large one: 112 / 300 us with
+// 16,385 groups, 237 / 396 with 131,072, 440 / 458 with 262,144: the searches
+// grow with groups x chunks, and the columns cross the link at half the
+// speed of a copy.
+constexpr uint64_t kSmallCap = 1 << 19;
 constexpr int kThreads = 256;
+// Slots up to which every key is compared with every other (8192 groups at
+// load 1/2); more are sorted by chunks. Whole group-by calls on B200,
+// comparing / by chunks of 2048: 72 / 85 us with 100 groups, 81 / 96 with
+// 4,099, 97 / 104 with 8,000, 117 / 107 with 12,000, 132 / 111 with 16,384.
+// (Chunks of 512: 91 with 4,099, but 370 where 2048 take 233, at 131,072.)
+constexpr uint64_t kFewCap = 1 << 14;
+constexpr unsigned kRankSplit = 16;  // CTAs that share the ranking of a tile of few keys
+constexpr unsigned kChunk = 2048;    // keys per CTA of a sorted chunk
+constexpr unsigned kChunkThreads = kChunk / 2;
 constexpr int kItems = 16;                    // keys per thread of a radix tile
 constexpr int kTile = kThreads * kItems;      // keys per CTA of a radix pass
 constexpr int kWarps = kThreads / 32;
@@ -130,17 +146,23 @@ __global__ void __launch_bounds__(kThreads) kCompact(TableArgs t, unsigned long 
     }
 }
 
-// Small tables: position = number of smaller keys (keys are distinct). Each
-// CTA places kThreads keys, reading all of them through shared memory.
-__global__ void __launch_bounds__(kThreads) kRank(const unsigned long long* n, const unsigned long long* __restrict__ keys,
-                                                  unsigned* __restrict__ order) {
+// Few keys: position = number of smaller keys. The kThreads keys of
+// blockIdx.x are compared with every kRankSplit-th tile of kThreads keys,
+// read through shared memory; the last of their CTAs to add its part places
+// them.
+__global__ void __launch_bounds__(kThreads) kRankAll(const unsigned long long* n,
+                                                     const unsigned long long* __restrict__ keys,
+                                                     const unsigned* __restrict__ slots, unsigned* ranks,
+                                                     unsigned* tickets, unsigned long long* __restrict__ keysOut,
+                                                     unsigned* __restrict__ slotsOut) {
     __shared__ unsigned long long tile[kThreads];
+    __shared__ bool last;
     const unsigned cnt = (unsigned)*n;
     const unsigned i = blockIdx.x * kThreads + threadIdx.x;
     if (blockIdx.x * kThreads >= cnt) return;
     const unsigned long long mine = i < cnt ? keys[i] : 0ull;
     unsigned rank = 0;
-    for (unsigned b = 0; b < cnt; b += kThreads) {
+    for (unsigned b = blockIdx.y * kThreads; b < cnt; b += kRankSplit * kThreads) {
         // past the end the tile holds the largest word, smaller than no key
         tile[threadIdx.x] = b + threadIdx.x < cnt ? keys[b + threadIdx.x] : ~0ull;
         __syncthreads();
@@ -148,21 +170,101 @@ __global__ void __launch_bounds__(kThreads) kRank(const unsigned long long* n, c
         for (int j = 0; j < kThreads; ++j) rank += tile[j] < mine;
         __syncthreads();
     }
-    if (i < cnt) order[rank] = i;
+    if (i < cnt && rank) atomicAdd(ranks + i, rank);
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) last = atomicAdd(tickets + blockIdx.x, 1u) == kRankSplit - 1u;
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    if (i < cnt) {
+        const unsigned r = __ldcg(ranks + i);
+        keysOut[r] = mine;
+        slotsOut[r] = slots[i];
+    }
+}
+
+// More keys, first of two launches: each CTA sorts kChunk keys with their
+// slots (bitonic, in shared memory; the keys are distinct). Past the end
+// chunks hold the largest word, after a key equal to it.
+__global__ void __launch_bounds__(kChunkThreads) kChunkSort(const unsigned long long* n,
+                                                       const unsigned long long* __restrict__ keys,
+                                                       const unsigned* __restrict__ slots,
+                                                       unsigned long long* __restrict__ chunkKeys,
+                                                       unsigned* __restrict__ chunkSlots) {
+    __shared__ unsigned long long k[kChunk];
+    __shared__ unsigned short x[kChunk];
+    const unsigned cnt = (unsigned)*n, b = blockIdx.x * kChunk;
+    if (b >= cnt) return;
+#pragma unroll
+    for (unsigned u = threadIdx.x; u < kChunk; u += kChunkThreads) {
+        k[u] = b + u < cnt ? keys[b + u] : ~0ull;
+        x[u] = (unsigned short)u;
+    }
+    for (unsigned size = 2; size <= kChunk; size *= 2)
+        for (unsigned d = size / 2; d > 0; d /= 2) {
+            __syncthreads();
+            const unsigned l = 2 * threadIdx.x - (threadIdx.x & (d - 1)), r = l + d;
+            const unsigned long long kl = k[l], kr = k[r];
+            const unsigned short xl = x[l], xr = x[r];
+            const bool swapped = kl > kr || (kl == kr && xl > xr);
+            if (swapped == ((l & size) == 0u)) {
+                k[l] = kr;
+                k[r] = kl;
+                x[l] = xr;
+                x[r] = xl;
+            }
+        }
+    __syncthreads();
+#pragma unroll
+    for (unsigned u = threadIdx.x; u < kChunk; u += kChunkThreads) {
+        chunkKeys[b + u] = k[u];
+        if (b + u < cnt) chunkSlots[b + u] = slots[b + x[u]];
+    }
+}
+
+// Second: a key's position is its place in its own chunk plus, for every
+// other chunk, the number of smaller keys there (binary searches, four
+// chunks' at a time so that their loads overlap).
+__global__ void __launch_bounds__(kThreads) kRank(const unsigned long long* n,
+                                                  const unsigned long long* __restrict__ chunkKeys,
+                                                  const unsigned* __restrict__ chunkSlots,
+                                                  unsigned long long* __restrict__ keys, unsigned* __restrict__ slots) {
+    const unsigned cnt = (unsigned)*n, i = blockIdx.x * kThreads + threadIdx.x;
+    if (i >= cnt) return;
+    const unsigned long long mine = chunkKeys[i];
+    const unsigned chunks = (cnt + kChunk - 1) / kChunk, own = i / kChunk;
+    unsigned rank = i % kChunk;
+    for (unsigned c = 0; c < chunks; c += 4) {
+        unsigned p[4] = {0u, 0u, 0u, 0u};
+        const unsigned long long* a[4];
+#pragma unroll
+        for (unsigned u = 0; u < 4; ++u) a[u] = chunkKeys + (c + u < chunks ? c + u : own) * kChunk;
+#pragma unroll
+        for (unsigned d = kChunk / 2; d > 0; d /= 2)
+#pragma unroll
+            for (unsigned u = 0; u < 4; ++u) p[u] += a[u][p[u] + d - 1] < mine ? d : 0u;
+#pragma unroll
+        for (unsigned u = 0; u < 4; ++u) {
+            p[u] += a[u][p[u]] < mine;
+            if (c + u < chunks && c + u != own) rank += p[u];
+        }
+    }
+    keys[rank] = mine;
+    slots[rank] = chunkSlots[i];
 }
 
 // Small tables: the columns in order, written straight into the mapped host
 // block: out[0] holds the group count, column c starts at out[1 + c * n].
 __global__ void __launch_bounds__(kThreads) kSmallOut(TableArgs t, const unsigned long long* n,
                                                       const unsigned long long* __restrict__ keys,
-                                                      const unsigned* __restrict__ slots,
-                                                      const unsigned* __restrict__ order, long long* out) {
+                                                      const unsigned* __restrict__ slots, long long* out) {
     const unsigned cnt = (unsigned)*n;
     const unsigned r = blockIdx.x * kThreads + threadIdx.x;
     if (r == 0) out[0] = cnt;
     if (r >= cnt) return;
-    const unsigned i = order ? order[r] : r, s = slots[i];
-    out[1 + r] = (long long)(keys[i] ^ 0x8000000000000000ull);
+    const unsigned s = slots[r];
+    out[1 + r] = (long long)(keys[r] ^ 0x8000000000000000ull);
     for (int a = 0; a < t.nAggs; ++a) out[1 + (unsigned long long)(1 + a) * cnt + r] = (long long)slotAgg(t, s, a);
 }
 
@@ -383,6 +485,80 @@ GroupWorkspace::~GroupWorkspace() {
     if (head) cudaFreeHost(head);
 }
 
+namespace {
+
+TableArgs tableArgs(const GroupTable& gt) {
+    TableArgs t{};
+    t.keys = gt.keys;
+    t.cap = gt.cap;
+    t.nAggs = gt.nAggs;
+    t.keyBytes = gt.keyBytes;
+    t.packedStride = gt.packedStride;
+    for (int a = 0; a < gt.nAggs && !gt.packedStride; a++) t.aggs[a] = static_cast<const unsigned long long*>(gt.aggs[a]);
+    return t;
+}
+
+unsigned scanGrid(uint64_t cap) { return (unsigned)std::min<uint64_t>((cap + kThreads - 1) / kThreads, 148 * 8); }
+
+size_t at256(size_t v) { return (v + 255) & ~size_t(255); }
+
+}  // namespace
+
+bool enqueueSmallGroups(const GroupTable& gt, bool sorted, GroupWorkspace& ws, cudaStream_t stream,
+                        std::shared_ptr<HostBlock>& host, std::string& error) {
+    error.clear();
+    if (gt.nAggs < 1 || gt.nAggs > GroupTable::kMaxAggs || gt.cap == 0 || gt.cap > kSmallCap) return false;
+    auto blk = hostBlock((1 + (1 + gt.nAggs) * (size_t)gt.cap) * 8);
+    void* mapped = nullptr;
+    if (!blk->pinned || cudaHostGetDevicePointer(&mapped, blk->ptr, 0) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    const unsigned blocks = (unsigned)((gt.cap + kThreads - 1) / kThreads);
+    // few keys: counters and ranks that start at 0, beside the group count;
+    // more: whole chunks of keys and slots
+    const bool few = gt.cap <= kFewCap;
+    const unsigned chunks = (unsigned)((gt.cap + kChunk - 1) / kChunk);
+    const size_t oTickets = 256, oRanks = oTickets + at256(4 * blocks), oKeys = few ? oRanks + at256(4 * gt.cap) : 256,
+                 oSlots = oKeys + at256(8 * gt.cap), oKeys2 = oSlots + at256(4 * gt.cap),
+                 n2 = few ? (size_t)gt.cap : (size_t)kChunk * chunks, oSlots2 = oKeys2 + at256(8 * n2);
+    if (!reserve(ws, oSlots2 + at256(4 * n2))) return false;
+    char* d = static_cast<char*>(ws.dev);
+    auto* n = reinterpret_cast<unsigned long long*>(d);
+    auto* keys = reinterpret_cast<unsigned long long*>(d + oKeys);
+    auto* slots = reinterpret_cast<unsigned*>(d + oSlots);
+    auto* keys2 = reinterpret_cast<unsigned long long*>(d + oKeys2);
+    auto* slots2 = reinterpret_cast<unsigned*>(d + oSlots2);
+    const TableArgs t = tableArgs(gt);
+    cudaError_t e = cudaMemsetAsync(d, 0, few ? oKeys : 256, stream);
+    if (e == cudaSuccess) {
+        kCompact<<<scanGrid(gt.cap), kThreads, 0, stream>>>(t, n, gt.cap, keys, slots);
+        if (sorted && few) {
+            kRankAll<<<dim3(blocks, kRankSplit), kThreads, 0, stream>>>(
+                n, keys, slots, reinterpret_cast<unsigned*>(d + oRanks), reinterpret_cast<unsigned*>(d + oTickets), keys2, slots2);
+            std::swap(keys, keys2);
+            std::swap(slots, slots2);
+        } else if (sorted) {
+            kChunkSort<<<chunks, kChunkThreads, 0, stream>>>(n, keys, slots, keys2, slots2);
+            kRank<<<blocks, kThreads, 0, stream>>>(n, keys2, slots2, keys, slots);
+        }
+        kSmallOut<<<blocks, kThreads, 0, stream>>>(t, n, keys, slots, static_cast<long long*>(mapped));
+        e = cudaGetLastError();
+    }
+    if (e != cudaSuccess) {
+        cudaStreamSynchronize(stream);  // nothing may still write the block
+        error = cudaWhy("group collection", e);
+        return false;
+    }
+    host = blk;
+    return true;
+}
+
+void smallGroups(const HostBlock& host, uint64_t& rows, const int64_t*& data) {
+    rows = *static_cast<const uint64_t*>(host.ptr);
+    data = static_cast<const int64_t*>(host.ptr) + 1;
+}
+
 bool collectGroups(const GroupTable& gt, bool sorted, GroupWorkspace& ws, cudaStream_t stream, uint64_t& rows,
                    const int64_t*& data, std::shared_ptr<HostBlock>& host, std::string& error) {
     error.clear();
@@ -394,46 +570,20 @@ bool collectGroups(const GroupTable& gt, bool sorted, GroupWorkspace& ws, cudaSt
         ws.head = nullptr;
         return false;
     }
-    TableArgs t{};
-    t.keys = gt.keys;
-    t.cap = gt.cap;
-    t.nAggs = gt.nAggs;
-    t.keyBytes = gt.keyBytes;
-    t.packedStride = gt.packedStride;
-    for (int a = 0; a < gt.nAggs && !gt.packedStride; a++) t.aggs[a] = static_cast<const unsigned long long*>(gt.aggs[a]);
-    const unsigned scanBlocks = (unsigned)std::min<uint64_t>((gt.cap + kThreads - 1) / kThreads, 148 * 8);
+    const TableArgs t = tableArgs(gt);
+    const unsigned scanBlocks = scanGrid(gt.cap);
     const int ncols = 1 + gt.nAggs;
-    auto at256 = [](size_t v) { return (v + 255) & ~size_t(255); };
     auto fail = [&](const char* what, cudaError_t e) {
         error = cudaWhy(what, e);
         return false;
     };
     cudaError_t e;
-    if (gt.cap <= kSmallCap) {
-        auto blk = hostBlock((1 + ncols * (size_t)gt.cap) * 8);
-        void* mapped = nullptr;
-        if (blk->pinned && cudaHostGetDevicePointer(&mapped, blk->ptr, 0) == cudaSuccess) {
-            const size_t oKeys = 256, oSlots = oKeys + at256(8 * gt.cap), oOrder = oSlots + at256(4 * gt.cap);
-            if (!reserve(ws, oOrder + at256(4 * gt.cap))) return false;
-            char* d = static_cast<char*>(ws.dev);
-            auto* n = reinterpret_cast<unsigned long long*>(d);
-            auto* keys = reinterpret_cast<unsigned long long*>(d + oKeys);
-            auto* slots = reinterpret_cast<unsigned*>(d + oSlots);
-            auto* order = sorted ? reinterpret_cast<unsigned*>(d + oOrder) : nullptr;
-            const unsigned blocks = (unsigned)((gt.cap + kThreads - 1) / kThreads);
-            if ((e = cudaMemsetAsync(n, 0, 8, stream)) != cudaSuccess) return fail("group collection", e);
-            kCompact<<<scanBlocks, kThreads, 0, stream>>>(t, n, gt.cap, keys, slots);
-            if (sorted) kRank<<<blocks, kThreads, 0, stream>>>(n, keys, order);
-            kSmallOut<<<blocks, kThreads, 0, stream>>>(t, n, keys, slots, order, static_cast<long long*>(mapped));
-            if ((e = cudaGetLastError()) != cudaSuccess || (e = cudaStreamSynchronize(stream)) != cudaSuccess)
-                return fail("group collection", e);
-            rows = *static_cast<uint64_t*>(blk->ptr);
-            data = static_cast<int64_t*>(blk->ptr) + 1;
-            host = blk;
-            return true;
-        }
-        cudaGetLastError();
+    if (enqueueSmallGroups(gt, sorted, ws, stream, host, error)) {
+        if ((e = cudaStreamSynchronize(stream)) != cudaSuccess) return fail("group collection", e);
+        smallGroups(*host, rows, data);
+        return true;
     }
+    if (!error.empty()) return false;
     if (!reserve(ws, 256)) return false;
     auto* head = static_cast<unsigned long long*>(ws.dev);
     ws.head[0] = 0;
