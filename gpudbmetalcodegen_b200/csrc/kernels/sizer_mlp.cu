@@ -41,7 +41,10 @@ constexpr int kThreads = 256;  // threads per CTA
 // 16-byte words of different banks. A thread owns 4 x SV outputs of each
 // layer (SV = TS / 16 neighbouring samples) and, in the weight gradients, 4 x 4
 // of a layer's matrix, which it keeps in registers over all tiles of its
-// CTA: one atomic per parameter and CTA instead of one per 32 samples.
+// CTA: one atomic per parameter and CTA instead of one per 32 samples. The
+// CTAs' sums meet in FP64: as many FP32 adds in a row as there are CTAs made
+// the gradients of 700 samples in tiles of 16 a third less accurate than those
+// in tiles of 32 (1.0e-7 of their norm against 7.5e-8).
 // Bound by shared-memory reads beside the FP32 adds (77 us of FMA at 100K
 // samples). B200, kernel alone, a 32-sample tile per CTA (weights read as
 // BF16 with all lanes in one bank, 30M atomics) -> this: training pass over
@@ -237,8 +240,8 @@ __device__ __forceinline__ void backW(const float* dOut, const float* in, float 
 template <int TS>
 __global__ void __launch_bounds__(kThreads, 2) mlpTrainStep(const __nv_bfloat16* __restrict__ wbf,
                                                             const float* __restrict__ X, const float* __restrict__ Y,
-                                                            int n, int total, float* __restrict__ grad,
-                                                            float* __restrict__ loss) {
+                                                            int n, int total, double* __restrict__ grad,
+                                                            double* __restrict__ loss) {
     using S = Smem<TS>;
     extern __shared__ __align__(16) unsigned char smraw[];
     S& sm = *reinterpret_cast<S*>(smraw);
@@ -295,23 +298,23 @@ __global__ void __launch_bounds__(kThreads, 2) mlpTrainStep(const __nv_bfloat16*
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
         const int j = jg + 16 * i;
-        atomicAdd(grad + kOffW1 + j * kIn + kg, g1[i][0]);
+        atomicAdd(grad + kOffW1 + j * kIn + kg, (double)g1[i][0]);
 #pragma unroll
         for (int c = 0; c < 4; ++c) {
-            atomicAdd(grad + kOffW2 + j * kH + kg + 16 * c, g2[i][c]);
-            atomicAdd(grad + kOffW3 + j * kH + kg + 16 * c, g3[i][c]);
+            atomicAdd(grad + kOffW2 + j * kH + kg + 16 * c, (double)g2[i][c]);
+            atomicAdd(grad + kOffW3 + j * kH + kg + 16 * c, (double)g3[i][c]);
         }
     }
     if (tid < kH) {
-        atomicAdd(grad + kOffB1 + tid, gb1);
-        atomicAdd(grad + kOffB2 + tid, gb2);
-        atomicAdd(grad + kOffB3 + tid, gb3);
+        atomicAdd(grad + kOffB1 + tid, (double)gb1);
+        atomicAdd(grad + kOffB2 + tid, (double)gb2);
+        atomicAdd(grad + kOffB3 + tid, (double)gb3);
     }
-    if (tid < kOut * kH) atomicAdd(grad + kOffW4 + tid, g4);
-    else if (tid < kOut * kH + kOut) atomicAdd(grad + kOffB4 + tid - kOut * kH, gb4);
+    if (tid < kOut * kH) atomicAdd(grad + kOffW4 + tid, (double)g4);
+    else if (tid < kOut * kH + kOut) atomicAdd(grad + kOffB4 + tid - kOut * kH, (double)gb4);
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) l += __shfl_xor_sync(0xffffffffu, l, o);
-    if ((tid & 31) == 0 && l != 0.0f) atomicAdd(loss, l / (float)(total * kOut));
+    if ((tid & 31) == 0 && l != 0.0f) atomicAdd(loss, (double)(l / (float)(total * kOut)));
 }
 
 template <int TS>
@@ -333,11 +336,11 @@ __global__ void __launch_bounds__(kThreads) mlpPredict(const __nv_bfloat16* __re
 
 // Adam on the FP32 master weights; refreshes the BF16 copy; clears grads.
 __global__ void adamStep(float* __restrict__ w, __nv_bfloat16* __restrict__ wbf, float* __restrict__ m,
-                         float* __restrict__ v, float* __restrict__ grad, float lr, float b1, float b2, float eps,
+                         float* __restrict__ v, double* __restrict__ grad, float lr, float b1, float b2, float eps,
                          float c1, float c2) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= kParams) return;
-    const float g = grad[i];
+    const float g = (float)grad[i];
     const float mi = b1 * m[i] + (1.0f - b1) * g;
     const float vi = b2 * v[i] + (1.0f - b2) * g * g;
     m[i] = mi;
@@ -345,7 +348,15 @@ __global__ void adamStep(float* __restrict__ w, __nv_bfloat16* __restrict__ wbf,
     const float wi = w[i] - lr * (mi / c1) / (sqrtf(vi / c2) + eps);
     w[i] = wi;
     wbf[i] = __float2bfloat16_rn(wi);
-    grad[i] = 0.0f;
+    grad[i] = 0.0;
+}
+
+// The gradients and the loss as FP32; clears the sums.
+__global__ void roundGrads(double* __restrict__ grad, float* __restrict__ out) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i > kParams) return;
+    out[i] = (float)grad[i];
+    grad[i] = 0.0;
 }
 
 __global__ void quantize(const float* __restrict__ w, __nv_bfloat16* __restrict__ wbf) {
@@ -367,7 +378,9 @@ __global__ void quantize(const float* __restrict__ w, __nv_bfloat16* __restrict_
 struct gpudb_sizer {
     int device = 0, numSMs = 148;
     cudaStream_t stream = nullptr;
-    float *w = nullptr, *m = nullptr, *v = nullptr, *grad = nullptr, *loss = nullptr;
+    float *w = nullptr, *m = nullptr, *v = nullptr;
+    double *grad = nullptr, *loss = nullptr;  // loss = grad + kParams
+    float* rounded = nullptr;                 // gradients and loss of gpudb_sizer_grads
     __nv_bfloat16* wbf = nullptr;
     float *X = nullptr, *Y = nullptr;
     int cap = 0;  // samples X/Y can hold
@@ -425,8 +438,9 @@ int gpudb_sizer_create(int device, uint64_t seed, gpudb_sizer** out) {
     SZ_CHECK(cudaMalloc(&s->w, sizeof(float) * kParams), GPUDB_E_ALLOC);
     SZ_CHECK(cudaMalloc(&s->m, sizeof(float) * kParams), GPUDB_E_ALLOC);
     SZ_CHECK(cudaMalloc(&s->v, sizeof(float) * kParams), GPUDB_E_ALLOC);
-    SZ_CHECK(cudaMalloc(&s->grad, sizeof(float) * kParams), GPUDB_E_ALLOC);
-    SZ_CHECK(cudaMalloc(&s->loss, sizeof(float)), GPUDB_E_ALLOC);
+    SZ_CHECK(cudaMalloc(&s->grad, sizeof(double) * (kParams + 1)), GPUDB_E_ALLOC);
+    s->loss = s->grad + kParams;
+    SZ_CHECK(cudaMalloc(&s->rounded, sizeof(float) * (kParams + 1)), GPUDB_E_ALLOC);
     SZ_CHECK(cudaMalloc(&s->wbf, sizeof(__nv_bfloat16) * kParams), GPUDB_E_ALLOC);
     // He-uniform initialisation on the host (seeded), biases zero
     std::vector<float> w(kParams, 0.0f);
@@ -443,7 +457,7 @@ int gpudb_sizer_create(int device, uint64_t seed, gpudb_sizer** out) {
     SZ_CHECK(cudaMemcpy(s->w, w.data(), sizeof(float) * kParams, cudaMemcpyHostToDevice), GPUDB_E_CUDA);
     SZ_CHECK(cudaMemset(s->m, 0, sizeof(float) * kParams), GPUDB_E_CUDA);
     SZ_CHECK(cudaMemset(s->v, 0, sizeof(float) * kParams), GPUDB_E_CUDA);
-    SZ_CHECK(cudaMemset(s->grad, 0, sizeof(float) * kParams), GPUDB_E_CUDA);
+    SZ_CHECK(cudaMemset(s->grad, 0, sizeof(double) * (kParams + 1)), GPUDB_E_CUDA);
     quantize<<<(kParams + 255) / 256, 256, 0, s->stream>>>(s->w, s->wbf);
     SZ_CHECK(cudaStreamSynchronize(s->stream), GPUDB_E_CUDA);
     *out = s.release();
@@ -454,7 +468,7 @@ void gpudb_sizer_free(gpudb_sizer* s) {
     if (!s) return;
     cudaSetDevice(s->device);
     if (s->stream) cudaStreamSynchronize(s->stream);
-    for (void* p : {(void*)s->w, (void*)s->m, (void*)s->v, (void*)s->grad, (void*)s->loss, (void*)s->wbf, (void*)s->X,
+    for (void* p : {(void*)s->w, (void*)s->m, (void*)s->v, (void*)s->grad, (void*)s->rounded, (void*)s->wbf, (void*)s->X,
                     (void*)s->Y})
         if (p) cudaFree(p);
     if (s->stream) cudaStreamDestroy(s->stream);
@@ -487,14 +501,13 @@ int gpudb_sizer_grads(gpudb_sizer* s, const float* X, const float* Y, int n, flo
     SZ_CHECK(cudaMemcpyAsync(s->X, X, sizeof(float) * (size_t)n * kIn, cudaMemcpyHostToDevice, s->stream), GPUDB_E_CUDA);
     SZ_CHECK(cudaMemcpyAsync(s->Y, Y, sizeof(float) * (size_t)n * kOut, cudaMemcpyHostToDevice, s->stream),
              GPUDB_E_CUDA);
-    SZ_CHECK(cudaMemsetAsync(s->grad, 0, sizeof(float) * kParams, s->stream), GPUDB_E_CUDA);
-    SZ_CHECK(cudaMemsetAsync(s->loss, 0, sizeof(float), s->stream), GPUDB_E_CUDA);
+    SZ_CHECK(cudaMemsetAsync(s->grad, 0, sizeof(double) * (kParams + 1), s->stream), GPUDB_E_CUDA);
     if (int st = launchTrain(s, s->X, s->Y, n, n)) return st;
-    SZ_CHECK(cudaMemcpyAsync(grads_out, s->grad, sizeof(float) * kParams, cudaMemcpyDeviceToHost, s->stream),
+    roundGrads<<<kParams / 256 + 1, 256, 0, s->stream>>>(s->grad, s->rounded);
+    SZ_CHECK(cudaMemcpyAsync(grads_out, s->rounded, sizeof(float) * kParams, cudaMemcpyDeviceToHost, s->stream),
              GPUDB_E_CUDA);
     float l = 0;
-    SZ_CHECK(cudaMemcpyAsync(&l, s->loss, sizeof(float), cudaMemcpyDeviceToHost, s->stream), GPUDB_E_CUDA);
-    SZ_CHECK(cudaMemsetAsync(s->grad, 0, sizeof(float) * kParams, s->stream), GPUDB_E_CUDA);
+    SZ_CHECK(cudaMemcpyAsync(&l, s->rounded + kParams, sizeof(float), cudaMemcpyDeviceToHost, s->stream), GPUDB_E_CUDA);
     SZ_CHECK(cudaStreamSynchronize(s->stream), GPUDB_E_CUDA);
     if (loss_out) *loss_out = l;
     return GPUDB_OK;
@@ -524,7 +537,7 @@ int gpudb_sizer_train(gpudb_sizer* s, const float* X, const float* Y, int n, int
                  GPUDB_E_CUDA);
         SZ_CHECK(cudaMemcpyAsync(s->Y, py.data(), sizeof(float) * py.size(), cudaMemcpyHostToDevice, s->stream),
                  GPUDB_E_CUDA);
-        SZ_CHECK(cudaMemsetAsync(s->loss, 0, sizeof(float), s->stream), GPUDB_E_CUDA);
+        SZ_CHECK(cudaMemsetAsync(s->loss, 0, sizeof(double), s->stream), GPUDB_E_CUDA);
         int nb = 0;
         for (int off = 0; off < n; off += batch, nb++) {
             const int cur = std::min(batch, n - off);
@@ -540,10 +553,10 @@ int gpudb_sizer_train(gpudb_sizer* s, const float* X, const float* Y, int n, int
                                                                     eps, c1, c2);
         }
         SZ_CHECK(cudaGetLastError(), GPUDB_E_LAUNCH);
-        float l = 0;
-        SZ_CHECK(cudaMemcpyAsync(&l, s->loss, sizeof(float), cudaMemcpyDeviceToHost, s->stream), GPUDB_E_CUDA);
+        double l = 0;
+        SZ_CHECK(cudaMemcpyAsync(&l, s->loss, sizeof(double), cudaMemcpyDeviceToHost, s->stream), GPUDB_E_CUDA);
         SZ_CHECK(cudaStreamSynchronize(s->stream), GPUDB_E_CUDA);
-        last = nb ? l / (float)nb : 0.0f;  // mean of the batches' losses
+        last = nb ? (float)(l / nb) : 0.0f;  // mean of the batches' losses
     }
     if (final_loss) *final_loss = last;
     return GPUDB_OK;
