@@ -895,8 +895,17 @@ __global__ void __launch_bounds__(kSampleThreads) kSampleStats(const QDesc* qs, 
     }
 }
 
-// ---- collect: per-query result rows and their exclusive prefix (one CTA) ---
-__global__ void kResultRows(const QDesc* __restrict__ qs, int n, unsigned long long* rows, unsigned long long* offs) {
+// ---- a batch's last launch: what the host needs to know of it (one CTA) ----
+// Per-query result rows and their exclusive prefix, for kCollect and in the
+// pinned `host` (rows[n], offs[n + 1]), the error words, and zeroed cursors.
+// The host waits for the batch alone: asked for afterwards (a launch, two
+// copies and a wait more), they were 40 us of a 300 us batch of 11 queries.
+__global__ void kResultRows(const QDesc* __restrict__ qs, int n, unsigned long long* offs, unsigned long long* cursors,
+                            const unsigned* __restrict__ errs, unsigned long long* host, unsigned* errHost) {
+    unsigned long long* rowsHost = host;
+    unsigned long long* offsHost = host + n;
+    for (int i = threadIdx.x; i <= n; i += blockDim.x) cursors[i] = 0ull;
+    for (int i = threadIdx.x; i < n; i += blockDim.x) errHost[i] = errs[i];
     __shared__ unsigned long long carry;
     __shared__ unsigned long long wsum[32];
     if (threadIdx.x == 0) carry = 0;
@@ -907,7 +916,7 @@ __global__ void kResultRows(const QDesc* __restrict__ qs, int n, unsigned long l
         if (i < n) {
             const QDesc& q = qs[i];
             r = q.tmpl == GPUDB_TPL_GROUPBY ? *q.nslots : q.tmpl == GPUDB_TPL_TOPK ? *q.topk_n : 1ull;
-            rows[i] = r;
+            rowsHost[i] = r;
         }
         unsigned long long x = r;  // inclusive warp scan
         for (int o = 1; o < 32; o <<= 1) {
@@ -918,16 +927,16 @@ __global__ void kResultRows(const QDesc* __restrict__ qs, int n, unsigned long l
         __syncthreads();
         unsigned long long before = carry;
         for (int w = 0; w < (int)(threadIdx.x >> 5); ++w) before += wsum[w];
-        if (i < n) offs[i] = before + x - r;
+        if (i < n) offsHost[i] = offs[i] = before + x - r;
         __syncthreads();
         if (threadIdx.x == blockDim.x - 1) carry = before + x;
         __syncthreads();
     }
-    if (threadIdx.x == 0) offs[n] = carry;
+    if (threadIdx.x == 0) offsHost[n] = offs[n] = carry;
 }
 
 // ---- collect: compaction of every query's rows into one packed buffer ------
-// `cursor`: one zeroed position counter per query (group rows come in no order).
+// `counter`, `cursor`: zero; one position counter per query (group rows come in no order).
 __global__ void __launch_bounds__(256) kCollect(const QDesc* __restrict__ qs, WorkList wl, unsigned long long* counter,
                                                 unsigned long long* cursor, const unsigned long long* __restrict__ offs,
                                                 long long* __restrict__ out) {
@@ -1052,9 +1061,9 @@ struct gpudb_batch {
     std::vector<QDesc> desc;
     DeviceBuf arena;  // zero-initialised per execution
     size_t zeroBytes = 0;
-    DeviceBuf scratch;  // never initialised: slot lists, top-k partials
+    DeviceBuf scratch;  // never initialised: result offsets and cursors, top-k partials
     DeviceBuf meta;     // descriptors + work lists
-    DeviceBuf stats, sample, collect;
+    DeviceBuf stats, collect;
     QDesc* dDesc = nullptr;
     WorkList wlBuild{}, wlAgg{}, wlGroup{}, wlScan{}, wlStats{}, wlCollect{};
     // rows per work item of each list: the tuning's, or fewer when the batch
@@ -1064,14 +1073,19 @@ struct gpudb_batch {
     int nTopk = 0;
     unsigned long long* counters = nullptr;  // work counters (first words of the arena)
     unsigned* errs = nullptr;                // one error word per query (behind the counters)
-    unsigned* errHost = nullptr;             // pinned copy of them
-    size_t errCap = 0;
+    unsigned long long* resOffs = nullptr;   // result offsets [n + 1]
+    unsigned long long* cursors = nullptr;   // kCollect's work counter and the queries' positions
+    bool cursorsZero = false;
+    // pinned, written by the kernels: rows[n] and offsets[n + 1] of the last
+    // execution, its error words, and the sample statistics
+    unsigned long long* resHost = nullptr;
+    unsigned* errHost = nullptr;
+    unsigned long long* sampleHost = nullptr;
+    size_t hostCap = 0;  // queries
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t graphExec = nullptr;
     bool dirty = true;
-    // rows per query, their offsets and total of the last execution, once a
-    // collect has asked for them (their device copies stay in `collect`)
-    std::vector<unsigned long long> resultRows;
+    bool executed = false;  // resHost holds the last execution's rows
     long long lastLaunches = 0;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     cudaEvent_t evStage[GPUDB_BATCH_STAGES + 1] = {};
@@ -1098,7 +1112,7 @@ int plan(gpudb_batch* b) {
     size_t z = al256(8 * 8);  // work counters
     const size_t zErr = z;
     z += al256(4 * (size_t)n);
-    size_t sc = 0;
+    size_t sc = al256(8 * (2 * (size_t)n + 2));  // offsets, cursors
     std::vector<size_t> zOff(n), sOff(n);
     std::vector<unsigned long long> caps(n, 0);
     std::vector<long long> tkChunks(n, 0);
@@ -1120,12 +1134,14 @@ int plan(gpudb_batch* b) {
         z = al256(z);
     }
     if (int st = b->arena.reserve(z, b->stream)) return st;
-    if (int st = b->scratch.reserve(std::max<size_t>(sc, 256), b->stream)) return st;
+    if (int st = b->scratch.reserve(sc, b->stream)) return st;
     b->zeroBytes = z;
     char* zb = static_cast<char*>(b->arena.p);
     char* sb = static_cast<char*>(b->scratch.p);
     b->counters = reinterpret_cast<unsigned long long*>(zb);
     b->errs = reinterpret_cast<unsigned*>(zb + zErr);
+    b->resOffs = reinterpret_cast<unsigned long long*>(sb);
+    b->cursors = b->resOffs + n + 1;
     b->desc.assign(n, QDesc{});
     std::vector<int> lBuild, lAgg, lGroup, lTopk, lAll(n), lCollect;
     std::vector<long long> pBuild{0}, pAgg{0}, pGroup{0}, pScan{0}, pAll{0}, pCollect{0};
@@ -1256,17 +1272,20 @@ int plan(gpudb_batch* b) {
     b->wlCollect = wl(oC, lCollect.size());
     b->dTopk = reinterpret_cast<int*>(m + oTop);
     b->nTopk = (int)lTopk.size();
-    if ((size_t)n > b->errCap) {
-        if (b->errHost) cudaFreeHost(b->errHost);
-        b->errHost = nullptr;
-        b->errCap = 0;
+    if ((size_t)n > b->hostCap) {
+        if (b->resHost) cudaFreeHost(b->resHost);
+        b->resHost = nullptr;
+        b->hostCap = 0;
         const size_t cap = std::max<size_t>(4096, 2 * (size_t)n);
-        B_CHECK(cudaHostAlloc((void**)&b->errHost, sizeof(unsigned) * cap, cudaHostAllocDefault), GPUDB_E_ALLOC);
-        b->errCap = cap;
+        B_CHECK(cudaHostAlloc((void**)&b->resHost, 8 * (2 * cap + 1) + 32 * cap + 4 * cap, cudaHostAllocDefault),
+                GPUDB_E_ALLOC);
+        b->sampleHost = b->resHost + 2 * cap + 1;
+        b->errHost = reinterpret_cast<unsigned*>(b->sampleHost + 4 * cap);
+        b->hostCap = cap;
     }
     B_CHECK(cudaStreamSynchronize(b->stream), GPUDB_E_CUDA);
     dropGraph(b);
-    b->resultRows.clear();
+    b->executed = false;
     b->dirty = false;
     return GPUDB_OK;
 }
@@ -1326,10 +1345,11 @@ int enqueue(gpudb_batch* b, bool stages) {
     }
     mark(6);
     B_CHECK(cudaGetLastError(), GPUDB_E_LAUNCH);
-    // per-query error words -> pinned host copy
-    if (n)
-        B_CHECK(cudaMemcpyAsync(b->errHost, b->errs, sizeof(unsigned) * n, cudaMemcpyDeviceToHost, b->stream),
-                GPUDB_E_CUDA);
+    if (n) {
+        kResultRows<<<1, 1024, 0, b->stream>>>(b->dDesc, n, b->resOffs, b->cursors, b->errs, b->resHost, b->errHost);
+        B_CHECK(cudaGetLastError(), GPUDB_E_LAUNCH);
+        launches++;
+    }
     b->lastLaunches = launches;
     return GPUDB_OK;
 }
@@ -1396,9 +1416,9 @@ void gpudb_batch_free(gpudb_batch* b) {
     cudaSetDevice(b->device);
     if (b->stream) cudaStreamSynchronize(b->stream);
     dropGraph(b);
-    for (DeviceBuf* d : {&b->arena, &b->scratch, &b->meta, &b->stats, &b->sample, &b->collect}) d->release(b->stream);
+    for (DeviceBuf* d : {&b->arena, &b->scratch, &b->meta, &b->stats, &b->collect}) d->release(b->stream);
     if (b->stream) cudaStreamSynchronize(b->stream);
-    if (b->errHost) cudaFreeHost(b->errHost);
+    if (b->resHost) cudaFreeHost(b->resHost);
     if (b->ev0) cudaEventDestroy(b->ev0);
     if (b->ev1) cudaEventDestroy(b->ev1);
     for (auto& e : b->evStage)
@@ -1511,7 +1531,7 @@ int gpudb_batch_execute(gpudb_batch* b, int use_graph, double* ms, uint32_t* err
     if (b->dirty)
         if (int st = plan(b)) return st;
     const int n = (int)b->queries.size();
-    b->resultRows.clear();
+    b->executed = false;
     B_CHECK(cudaEventRecord(b->ev0, b->stream), GPUDB_E_CUDA);
     if (use_graph) {
         if (!b->graphExec) {
@@ -1543,6 +1563,8 @@ int gpudb_batch_execute(gpudb_batch* b, int use_graph, double* ms, uint32_t* err
         }
         b->stagesValid = true;
     }
+    b->executed = true;
+    b->cursorsZero = true;
     if (errors && n) std::memcpy(errors, b->errHost, sizeof(unsigned) * n);
     return GPUDB_OK;
 }
@@ -1604,14 +1626,11 @@ int gpudb_batch_features(gpudb_batch* b, float* f, double* ms) {
         if (int st = plan(b)) return st;
     const int n = (int)b->queries.size();
     if (n == 0) return GPUDB_OK;
-    if (int st = b->sample.reserve(32 * (size_t)n, b->stream)) return st;
-    unsigned long long* out = static_cast<unsigned long long*>(b->sample.p);
+    const unsigned long long* h = b->sampleHost;
     B_CHECK(cudaEventRecord(b->ev0, b->stream), GPUDB_E_CUDA);
-    kSampleStats<<<n, kSampleThreads, kSampleSmem, b->stream>>>(b->dDesc, out);
+    kSampleStats<<<n, kSampleThreads, kSampleSmem, b->stream>>>(b->dDesc, b->sampleHost);
     B_CHECK(cudaGetLastError(), GPUDB_E_LAUNCH);
     B_CHECK(cudaEventRecord(b->ev1, b->stream), GPUDB_E_CUDA);
-    std::vector<unsigned long long> h(4 * (size_t)n);
-    B_CHECK(cudaMemcpyAsync(h.data(), out, 32 * (size_t)n, cudaMemcpyDeviceToHost, b->stream), GPUDB_E_CUDA);
     B_CHECK(cudaStreamSynchronize(b->stream), GPUDB_E_CUDA);
     if (ms) *ms = elapsed(b);
     for (int i = 0; i < n; i++) {
@@ -1661,45 +1680,31 @@ int gpudb_batch_collect(gpudb_batch* b, uint64_t* rows, void* host, uint64_t hos
         if (bytes_needed) *bytes_needed = 0;
         return GPUDB_OK;
     }
-    // rows[n] + offsets[n+1] + counter + cursors[n], then the packed result rows
-    const size_t head = al256(8 * (3 * (size_t)n + 2));
-    size_t maxRows = 0;
-    for (int i = 0; i < n; i++) {
-        const auto& q = b->queries[i];
-        maxRows += q.tmpl == GPUDB_TPL_GROUPBY ? (size_t)pow2ceil(2 * std::max<uint64_t>(q.groups, 1))
-                   : q.tmpl == GPUDB_TPL_TOPK  ? (size_t)kTopK
-                                               : 1;
+    if (!b->executed) {
+        gpudb::setThreadError("batch: collect before execute");
+        return GPUDB_E_INVALID;
     }
-    if (int st = b->collect.reserve(head + 24 * maxRows, b->stream)) return st;
-    unsigned long long* dRows = static_cast<unsigned long long*>(b->collect.p);
-    unsigned long long* dOffs = dRows + n;
-    unsigned long long* counter = dOffs + n + 1;
-    long long* out = reinterpret_cast<long long*>(static_cast<char*>(b->collect.p) + head);
-    B_CHECK(cudaEventRecord(b->ev0, b->stream), GPUDB_E_CUDA);
-    std::vector<unsigned long long>& h = b->resultRows;
-    if (h.empty()) {
-        kResultRows<<<1, 1024, 0, b->stream>>>(b->dDesc, n, dRows, dOffs);
-        B_CHECK(cudaGetLastError(), GPUDB_E_LAUNCH);
-        std::vector<unsigned long long> got(2 * (size_t)n + 1);
-        B_CHECK(cudaMemcpyAsync(got.data(), dRows, 8 * got.size(), cudaMemcpyDeviceToHost, b->stream), GPUDB_E_CUDA);
-        B_CHECK(cudaStreamSynchronize(b->stream), GPUDB_E_CUDA);
-        h = std::move(got);
-    }
-    const unsigned long long total = h[2 * (size_t)n];
+    const unsigned long long total = b->resHost[2 * (size_t)n];
     if (rows)
-        for (int i = 0; i < n; i++) rows[i] = h[i];
+        for (int i = 0; i < n; i++) rows[i] = b->resHost[i];
     if (bytes_needed) *bytes_needed = 24 * total;
-    if (host) {
-        if (host_bytes < 24 * total) {
-            gpudb::setThreadError("batch: collect buffer too small");
-            return GPUDB_E_INVALID;
-        }
-        B_CHECK(cudaMemsetAsync(counter, 0, 8 * ((size_t)n + 1), b->stream), GPUDB_E_CUDA);
-        kCollect<<<gridFor(b, (const void*)kCollect, 256), 256, 0, b->stream>>>(b->dDesc, b->wlCollect, counter,
-                                                                               counter + 1, dOffs, out);
-        B_CHECK(cudaGetLastError(), GPUDB_E_LAUNCH);
-        if (total) B_CHECK(cudaMemcpyAsync(host, out, 24 * total, cudaMemcpyDeviceToHost, b->stream), GPUDB_E_CUDA);
+    if (ms) *ms = 0.0;
+    if (!host) return GPUDB_OK;
+    if (host_bytes < 24 * total) {
+        gpudb::setThreadError("batch: collect buffer too small");
+        return GPUDB_E_INVALID;
     }
+    if (total == 0) return GPUDB_OK;
+    if (int st = b->collect.reserve(24 * total, b->stream)) return st;
+    long long* out = static_cast<long long*>(b->collect.p);
+    B_CHECK(cudaEventRecord(b->ev0, b->stream), GPUDB_E_CUDA);
+    if (!b->cursorsZero)
+        B_CHECK(cudaMemsetAsync(b->cursors, 0, 8 * ((size_t)n + 1), b->stream), GPUDB_E_CUDA);
+    b->cursorsZero = false;
+    kCollect<<<gridFor(b, (const void*)kCollect, 256), 256, 0, b->stream>>>(b->dDesc, b->wlCollect, b->cursors,
+                                                                           b->cursors + 1, b->resOffs, out);
+    B_CHECK(cudaGetLastError(), GPUDB_E_LAUNCH);
+    B_CHECK(cudaMemcpyAsync(host, out, 24 * total, cudaMemcpyDeviceToHost, b->stream), GPUDB_E_CUDA);
     B_CHECK(cudaEventRecord(b->ev1, b->stream), GPUDB_E_CUDA);
     B_CHECK(cudaEventSynchronize(b->ev1), GPUDB_E_CUDA);
     if (ms) *ms = elapsed(b);
