@@ -3,8 +3,8 @@
 //
 // What it replaces: copying the whole table to pageable host memory, one
 // host pass over its slots, a host sort and a row object per group. Measured
-// on B200, whole calls: a hash join with 2^20 keys 350 ms before, 1.71 ms
-// now (0.8 ms of it the join's kernels, 0.5 ms the 25 MB over the link); a
+// on B200, whole calls: a hash join with 2^20 keys 350 ms before, 1.17 ms
+// now (0.34 ms of it the join's kernels, 0.46 ms the 25 MB over the link); a
 // group-by with 4,099 groups 788 us before, 80 us now.
 //
 // Tables of at most kSmallCap slots follow the query's own kernels without a
@@ -49,8 +49,11 @@ constexpr uint64_t kFewCap = 1 << 14;
 constexpr unsigned kRankSplit = 16;  // CTAs that share the ranking of a tile of few keys
 constexpr unsigned kChunk = 2048;    // keys per CTA of a sorted chunk
 constexpr unsigned kChunkThreads = kChunk / 2;
-constexpr int kItems = 16;                    // keys per thread of a radix tile
-constexpr int kTile = kThreads * kItems;      // keys per CTA of a radix pass
+// Keys per thread of a radix tile: a pass waits for memory and ranks, so more
+// and smaller CTAs win. Whole calls on B200 with 16 / 8 / 4: 474 / 429 / 405
+// us at 300,000 groups, 886 / 876 / 853 at 1M, 3,078 / 2,968 / 2,967 at 4M.
+constexpr int kItems = 4;
+constexpr int kTile = kThreads * kItems;  // keys per CTA of a radix pass
 constexpr int kWarps = kThreads / 32;
 
 struct TableArgs {

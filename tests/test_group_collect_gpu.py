@@ -1,7 +1,7 @@
 """Collecting a hash aggregate's groups on the device (compaction, key order,
-dense columns) against numpy, at the sizes where a path or a tile ends: the
-rank sort serves tables of up to 32768 slots (16384 groups at load 1/2), the
-radix sort works in tiles of 4096 keys and skips digits no two keys differ in."""
+dense columns) against numpy, at the sizes where a path or a tile ends: keys
+are compared in tiles of 256 or sorted by chunks of 2048, and past 2^19 slots
+sorted digit by digit, skipping digits no two keys differ in."""
 import gc
 
 import numpy as np

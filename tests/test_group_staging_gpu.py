@@ -2,7 +2,7 @@
 warmed-up, uncollected, failing and growing runs must each return their own
 groups. Up to 2^14 slots (8192 groups at load 1/2) keys are compared in tiles
 of 256, up to 2^19 they are sorted by chunks of 2048; larger tables are
-collected after the run."""
+collected after the run, by radix passes over tiles of 1024."""
 import numpy as np
 import pytest
 
@@ -23,7 +23,7 @@ def check(got, keys, scale):
 
 
 @pytest.mark.parametrize("tune", ["", "layout=packed"])
-@pytest.mark.parametrize("groups", [1, 255, 256, 257, 4097, 8192, 8193, 10_240, 131_073, 262_144, 262_145])
+@pytest.mark.parametrize("groups", [1, 255, 256, 257, 4097, 8192, 8193, 10_240, 131_073, 262_144, 262_145, 263_168, 300_007])
 def test_each_run_returns_its_own_groups(groups, tune):
     rng = np.random.default_rng(groups)
     with Context(0) as ctx:
