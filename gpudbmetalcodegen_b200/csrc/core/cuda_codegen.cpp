@@ -316,6 +316,7 @@ std::string CudaCodegen::print() {
     if (phases_.size() > kMaxPhases) throw std::runtime_error("CudaCodegen::print: too many phases");
     for (size_t pi = 0; pi < phases_.size(); pi++) {
         assignArgIndices(phases_[pi]);
+        phases_[pi].writesStart = true;
         const auto& ph = phases_[pi];
         out << "\n// === Phase " << pi << ": " << ph.name << " ===\n";
         out << generateSignature(ph) << " {\n";

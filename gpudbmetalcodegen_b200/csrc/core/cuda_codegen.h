@@ -140,6 +140,7 @@ public:
         int maxThreadgroups = 0;
         bool cooperative = false;  // the blocks wait on one another: launched all resident
         bool isSingleThread = false;
+        bool writesStart = false;  // generated: the kernel writes its start time beside the error word
         int dynamicSmemBytes = 0;
         int tileRows = 0;
         int rowsPerThread = 1;

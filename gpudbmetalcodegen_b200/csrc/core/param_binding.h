@@ -42,7 +42,8 @@ enum class CudaParamKind {
     DeviceBuffer,    // T* (or const T*)             — executor-allocated scratch/output
     ConstantScalar,  // scalar by value              — registered with register_scalar_*
     ConstantData,    // const T* to uploaded host data
-    ErrorWord,       // unsigned*                    — device error word, always last
+    ErrorWord,       // unsigned*                    — device error word, always last; phase i writes its
+                     //                                start time (u64, ns) 8 + 8 i bytes behind it
     BufferLength,    // long long                    — element count of a named buffer
 };
 

@@ -48,7 +48,7 @@ CudaGenericExecutor::CudaGenericExecutor(int device) : device_(device) {
     // the error word's copy and the staging area share one pinned block
     GPUDB_CUDA_OR_THROW(cudaHostAlloc((void**)&stageHost_, kStageBytes + kErrBytes, cudaHostAllocDefault));
     errHost_ = reinterpret_cast<unsigned*>(stageHost_ + kStageBytes);
-    for (auto& e : events_) GPUDB_CUDA_OR_THROW(cudaEventCreate(&e));
+    ensureEvents(2);
     const DriverApi& api = driverApi();
     if (!api.loaded) throw std::runtime_error("CUDA driver API unavailable: " + api.error);
 }
@@ -61,8 +61,7 @@ CudaGenericExecutor::~CudaGenericExecutor() {
     for (auto& [_, b] : ownedColumns_)
         if (b.ptr) cudaFree(b.ptr);
     ownedColumns_.clear();
-    for (auto e : events_)
-        if (e) cudaEventDestroy(e);
+    for (auto e : events_) cudaEventDestroy(e);
     if (errWord_) cudaFree(errWord_);
     if (stageHost_) cudaFreeHost(stageHost_);
     if (stream_) cudaStreamDestroy(stream_);
@@ -337,6 +336,14 @@ GenericResult CudaGenericExecutor::collectResult(const CudaResultSchema& schema)
 // ---------------------------------------------------------------------------
 // launch preparation
 // ---------------------------------------------------------------------------
+void CudaGenericExecutor::ensureEvents(size_t n) {
+    while (events_.size() < n) {
+        cudaEvent_t e;
+        GPUDB_CUDA_OR_THROW(cudaEventCreate(&e));
+        events_.push_back(e);
+    }
+}
+
 bool CudaGenericExecutor::buildLaunch(const RuntimeCompiler::CompiledQuery& cq, const CudaCodegen::PhaseInfo& ph,
                                       Launch& l, std::string& error) {
     const DriverApi& api = driverApi();
@@ -536,7 +543,10 @@ int CudaGenericExecutor::execute(const RuntimeCompiler::CompiledQuery& cq,
     out.totalKernelTimeMs = 0.0;
 
     // Timed iterations record an event after the fills and one after the
-    // last kernel.
+    // last kernel; after every kernel where one does not write its start.
+    bool starts = true;
+    for (int p = first; p < last; p++) starts = starts && phases[p].writesStart;
+    if (!starts) ensureEvents(nl + 1);
     auto launchAll = [&](bool timed) -> bool {
         if (fillBuffers(fills, stream_) != cudaSuccess) {
             error = "buffer fill failed";
@@ -552,6 +562,7 @@ int CudaGenericExecutor::execute(const RuntimeCompiler::CompiledQuery& cq,
                 l.cooperative
                     ? api.cuLaunchCooperativeKernel(l.fn, l.grid, 1, 1, l.block, 1, 1, l.smem, (CUstream)stream_, args.data())
                     : api.cuLaunchKernel(l.fn, l.grid, 1, 1, l.block, 1, 1, l.smem, (CUstream)stream_, args.data(), nullptr);
+            if (timed && !starts && i + 1 < nl) cudaEventRecord(events_[2 + i], stream_);
             if (r != CUDA_SUCCESS) {
                 error = "launch of '" + l.name + "' failed: " + cuErrorString(r);
                 return false;
@@ -626,7 +637,7 @@ int CudaGenericExecutor::execute(const RuntimeCompiler::CompiledQuery& cq,
     unsigned bits = 0;
     auto wait = [&](int iter, const char* what) -> bool {
         if (iter == total - 1 && !stage) stageSchema_ = nullptr;
-        if (!enqueueTail(iter == total - 1, phases.size())) {
+        if (!enqueueTail(iter == total - 1, starts ? (size_t)last : 0)) {
             error = "cannot read the device error word";
             return false;
         }
@@ -657,7 +668,13 @@ int CudaGenericExecutor::execute(const RuntimeCompiler::CompiledQuery& cq,
             const uint64_t* start = reinterpret_cast<const uint64_t*>(errHost_) + 1 + first;
             double rest = ms;
             for (size_t i = 0; i + 1 < nl; i++) {
-                const double t = std::min(rest, start[i + 1] > start[i] ? (start[i + 1] - start[i]) * 1e-6 : 0.0);
+                double t = 0.0;
+                if (starts) {
+                    if (start[i + 1] > start[i]) t = std::min(rest, (start[i + 1] - start[i]) * 1e-6);
+                } else {
+                    cudaEventElapsedTime(&ms, events_[i ? 1 + i : 0], events_[2 + i]);
+                    t = std::min<double>(rest, ms);
+                }
                 out.phaseTimesMs[i] += t / measured;
                 rest -= t;
             }

@@ -13,8 +13,8 @@
 //     stream-ordered, the host synchronises once per execute(), and the
 //     error word and a small result come back under that same wait;
 //   * a run is timed by two CUDA events, its phases by the start time that
-//     each kernel writes beside the error word (the reference's GPU
-//     timestamps);
+//     each generated kernel writes beside the error word (the reference's
+//     GPU timestamps), or by events where a kernel is the caller's own;
 //   * launch = min(work, SMs x occupancy) persistent CTAs, with the
 //     dynamic shared memory each phase declares (TMA ring, smem tables);
 //   * the device error word is cleared before and read after each run;
@@ -174,7 +174,7 @@ private:
     std::map<std::pair<uint64_t, CUfunction>, int> carveoutSet_;
     // blocks per SM of (load id, function, block, dynamic shared memory)
     std::map<std::tuple<uint64_t, CUfunction, unsigned, unsigned>, int> occupancy_;
-    cudaEvent_t events_[2] = {nullptr, nullptr};  // around a timed iteration's kernels
+    std::vector<cudaEvent_t> events_;  // before and after a timed iteration's kernels, and between the callers' own
     // pinned copies of the buffers a result is decoded from
     struct Staged {
         std::string name;
@@ -198,6 +198,7 @@ private:
     std::unordered_set<std::string> seenOnce_;    // keys run once, eagerly, not captured yet
     static constexpr size_t kMaxSeen = 4096;
 
+    void ensureEvents(size_t n);
     bool allocateBuffers(const CudaCodegen::PhaseInfo& phase, std::string& error);
     bool buildLaunch(const RuntimeCompiler::CompiledQuery& cq, const CudaCodegen::PhaseInfo& phase, Launch& l,
                      std::string& error);

@@ -1,13 +1,19 @@
 """What a run reads back in one launch: its phases' start times, the error
 word and the result's small buffers, from none to more than one launch of 32."""
+import ctypes as C
+from pathlib import Path
+
 import numpy as np
 import pytest
 
 from gpudbmetalcodegen_b200 import Context
+from gpudbmetalcodegen_b200 import _lib
 from gpudbmetalcodegen_b200 import analyzed as A
 from gpudbmetalcodegen_b200 import workloads as W
 
 pytestmark = pytest.mark.gpu
+
+HEADER = Path(__file__).resolve().parent.parent / "gpudbmetalcodegen_b200" / "csrc" / "kernels" / "gpudb_device.cuh"
 
 
 @pytest.fixture(scope="module")
@@ -44,3 +50,33 @@ def test_many_result_buffers(ctx, naggs):
     q = int(fact["f_quantity"].astype(np.int64).sum())
     assert t.device_error == 0
     assert res.rows == [tuple(q * (j + 1) for j in range(naggs))]
+
+
+SPIN = r"""
+extern "C" __global__ void spin_100us(unsigned* gpudb_err) {
+    const unsigned long long t0 = gpudb_now_ns();
+    for (int i = 0; i < 1000000 && gpudb_now_ns() - t0 < 100000ull; ++i) {}
+}
+extern "C" __global__ void spin_300us(unsigned* gpudb_err) {
+    const unsigned long long t0 = gpudb_now_ns();
+    for (int i = 0; i < 1000000 && gpudb_now_ns() - t0 < 300000ull; ++i) {}
+}
+"""
+
+
+@pytest.mark.parametrize("warmup,measured", [(0, 1), (1, 3)])
+def test_hand_written_kernels_are_timed(ctx, warmup, measured):
+    """Kernels that write no start time: each phase lasts at least as long as
+    its loop, and not as long as both."""
+    lib = _lib.load()
+    src = HEADER.read_text() + SPIN
+    mod = C.c_void_p()
+    names = (C.c_char_p * 2)(b"spin_100us", b"spin_300us")
+    _lib.check(lib.gpudb_compile(ctx.handle, src.encode(), names, 2, C.byref(mod)), ctx.handle)
+    bind = (_lib.BindingDesc * 1)(_lib.BindingDesc(b"gpudb_err", _lib.PARAM_ERROR_WORD, b"unsigned", None, None, 1, 0, 0))
+    ph = (_lib.PhaseDesc * 2)(*(_lib.PhaseDesc(n, None, 32, 1, 0, 0, 0, 1, bind, 1) for n in names))
+    t = _lib.Timing()
+    _lib.check(lib.gpudb_execute(ctx.handle, mod, ph, 2, 0, 2, warmup, measured, C.byref(t)), ctx.handle)
+    lib.gpudb_module_free(mod)
+    assert 0.1 <= t.phase_ms[0] < 0.3 <= t.phase_ms[1] < 0.4
+    assert t.phase_ms[0] + t.phase_ms[1] == pytest.approx(t.total_ms, rel=1e-9)
