@@ -899,7 +899,7 @@ __global__ void __launch_bounds__(kSampleThreads) kSampleStats(const QDesc* qs, 
 // Per-query result rows and their exclusive prefix, for kCollect and in the
 // pinned `host` (rows[n], offs[n + 1]), the error words, and zeroed cursors.
 // The host waits for the batch alone: asked for afterwards (a launch, two
-// copies and a wait more), they were 40 us of a 300 us batch of 11 queries.
+// copies and a wait more), they were 40 us of a 300 us batch of four queries.
 __global__ void kResultRows(const QDesc* __restrict__ qs, int n, unsigned long long* offs, unsigned long long* cursors,
                             const unsigned* __restrict__ errs, unsigned long long* host, unsigned* errHost) {
     unsigned long long* rowsHost = host;

@@ -318,6 +318,21 @@ __global__ void __launch_bounds__(kThreads) kDigitScan(unsigned* __restrict__ co
     if (threadIdx.x == 0) totals[blockIdx.x] = carry;
 }
 
+// The lanes with the same 8-bit digit (of those that are `in`, or of the
+// others): nine ballots. A match-any per item instead: 1,185 us for a hash
+// join with 2^20 groups that takes 1,157, 857 / 831 for a group-by with 1M.
+__device__ __forceinline__ unsigned digitPeers(unsigned d, bool in) {
+    const unsigned m = __ballot_sync(0xffffffffu, in);
+    unsigned peers = in ? m : ~m;
+#pragma unroll
+    for (int b = 0; b < 8; ++b) {
+        const bool one = d >> b & 1u;
+        const unsigned v = __ballot_sync(0xffffffffu, one);
+        peers &= one ? v : ~v;
+    }
+    return peers;
+}
+
 // Stable scatter of a tile: each warp owns kItems * 32 consecutive pairs and
 // ranks equal digits by match-any, 32 at a time; the warps' counts then
 // become offsets from the digit's base.
@@ -353,8 +368,8 @@ __global__ void __launch_bounds__(kThreads) kDigitScatter(const unsigned long lo
 #pragma unroll
     for (int u = 0; u < kItems; ++u) {
         const bool in = b + u * 32u < n;
-        const unsigned dg = in ? (unsigned)(k[u] >> shift) & 255u : 256u;
-        const unsigned peers = __match_any_sync(0xffffffffu, dg);
+        const unsigned dg = (unsigned)(k[u] >> shift) & 255u;
+        const unsigned peers = digitPeers(dg, in);
         const unsigned before = in ? cnt[warp][dg] : 0u;
         __syncwarp();
         if (in && (int)lane == __ffs(peers) - 1) cnt[warp][dg] = before + __popc(peers);

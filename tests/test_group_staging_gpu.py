@@ -51,3 +51,23 @@ def test_a_failed_run_returns_nothing_and_the_next_one_its_own():
         keys = keys % 9
         load(ctx, keys, 3)
         check(ctx.run("template=groupby", arrays=True)[0], keys, 3)
+
+
+@pytest.mark.parametrize("groups", [700, 70_001])
+def test_replayed_graphs_return_the_same_groups(groups):
+    """Captured fills, kernels and, for the sorted form, a cooperative sort."""
+    keys = np.random.default_rng(5).permutation(np.arange(5 * groups, dtype=np.int64) % groups) * 31
+    with Context(0) as ctx:
+        ctx.register_symbol("zgroups", groups)
+        load(ctx, keys, 2)
+        ctx.set_use_graphs(True)
+        q, s = ctx.prepare("template=groupby"), ctx.prepare("template=groupby_sorted")
+        for _ in range(4):
+            check(ctx.run(q, arrays=True)[0], keys, 2)
+            got, t = ctx.run(s, collect=False)
+            n = int(ctx.read_buffer("gss_n", np.uint64, 1)[0])
+            assert t.device_error == 0 and n == groups
+            k, v = ctx.read_buffer("gss_out_k", np.int64, n), ctx.read_buffer("gss_out_v", np.int64, n)
+            uk, cnt = np.unique(keys, return_counts=True)
+            o = np.lexsort((uk, -(uk * cnt * 2)))
+            assert np.array_equal(k, uk[o]) and np.array_equal(v, (uk * cnt * 2)[o])
