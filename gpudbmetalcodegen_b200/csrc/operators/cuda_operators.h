@@ -639,8 +639,8 @@ private:
 // ------------------------------------------------------------------
 class CudaGroupSort : public CudaOperator {
 public:
-    static constexpr int kThreads = 512, kTile = 4096;         // GPUDB_RS_THREADS, GPUDB_RS_TILE
-    static constexpr int kSmemWords = 16 * 256 + 256 + 32;     // GPUDB_RS_SMEM_WORDS
+    static constexpr int kThreads = 512, kTile = 2048;         // GPUDB_RS_THREADS, GPUDB_RS_TILE
+    static constexpr int kSmemWords = 3 * kTile + 16 * 256 + 512 + 32;  // GPUDB_RS_SMEM_WORDS
     CudaGroupSort(const std::string& prefix, const std::string& countBuffer, const std::string& capacityExpr);
     // The dense input arrays (key, count, value).
     void setInput(const std::string& keys, const std::string& counts, const std::string& values);
